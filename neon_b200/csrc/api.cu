@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "cg_group.cuh"
 #include "host_driver.hpp"
 #include "nb2_internal.cuh"
 
@@ -238,6 +239,7 @@ int nb2_destroy(nb2_ctx* c) {
     if (!c) return NB2_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     release_graphs(c);
+    sell_release(c->sell);
     void* ptrs[] = {c->X,      c->conn,   c->brp,    c->bcol,   c->slot,      c->K64,
                     c->K32,    c->u,      c->u_old,  c->fint,   c->fext,      c->rhs,
                     c->du,     c->inc,    c->mask,   c->Ge,     c->Ke,        c->ep,

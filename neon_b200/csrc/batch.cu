@@ -21,6 +21,7 @@
 #include <string>
 #include <vector>
 
+#include "cg_group.cuh"
 #include "host_driver.hpp"
 #include "nb2_internal.cuh"
 
@@ -137,6 +138,7 @@ __global__ void __launch_bounds__(kThreads) k_b_init(Tables T, const double* __r
             S.thr[inst] = fmax(tol * tol * tot[0], DBL_MIN);
             S.rr[inst] = tot[1];
             S.rrcap[inst] = INFINITY;
+            S.beta[inst] = 0.0;
             S.absnew[inst] = tot[2];
             S.iters[inst] = 0;
             S.status[inst] = 0;
@@ -490,6 +492,7 @@ struct BatchState {
     std::vector<double> h_norms;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     float* dcomp = nullptr;    // FP32 K mode: the compensated diagonal's correction (n)
+    SellPlan* plan = nullptr;  // persistent PCG of this K (the context's; null: chunk kernels)
 
     Tables tables() const { return Tables{row0, row1, inst, first, count}; }
     Scalars scalars() const {
@@ -590,6 +593,10 @@ int batch_setup(nb2_ctx* c, const int* node_offsets, int ninst, int R, int lanes
     return NB2_OK;
 }
 
+bool any(const std::vector<int>& v) {
+    return std::any_of(v.begin(), v.end(), [](int x) { return x != 0; });
+}
+
 int upload_flags(nb2_ctx* c, int* d, const std::vector<int>& h) {
     NB2_CUDA(c, cudaMemcpyAsync(d, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice,
                                 c->stream));
@@ -631,6 +638,10 @@ int batch_pcg_start(nb2_ctx* c, BatchState* b, int mode, const double* rhs, doub
     k_b_init<double><<<b->nchunks, kThreads, 0, c->stream>>>(T, rhs, c->cg_x, c->cg_r, c->cg_p,
                                                               c->cg_inv, S, b->part, tol);
     c->launches += 2;
+    NB2_TRY(sell_plan(c, b->h_node_off, mode == kModeK64 ? 8 : 4, &b->plan));
+    if (b->plan && (mode == kModeK64 ? sell_fill(c, b->plan, c->K64, c->mask)
+                                     : sell_fill(c, b->plan, c->K32, c->mask)) != NB2_OK)
+        b->plan = nullptr;
     NB2_CUDA(c, cudaStreamSynchronize(c->stream));  // maxit's host vector is the caller's
     return NB2_OK;
 }
@@ -638,6 +649,43 @@ int batch_pcg_start(nb2_ctx* c, BatchState* b, int mode, const double* rhs, doub
 int batch_pcg_iterate(nb2_ctx* c, BatchState* b, int mode, int most, bool graphs) {
     const Tables T = b->tables();
     const Scalars S = b->scalars();
+    auto read_done = [&]() -> int {
+        NB2_CUDA(c, cudaMemcpyAsync(b->h_done.data(), S.done, sizeof(int) * b->ninst,
+                                    cudaMemcpyDeviceToHost, c->stream));
+        NB2_CUDA(c, cudaStreamSynchronize(c->stream));
+        return NB2_OK;
+    };
+    auto read_results = [&]() -> int {
+        NB2_CUDA(c, cudaMemcpyAsync(b->h_iters.data(), S.iters, sizeof(int) * b->ninst,
+                                    cudaMemcpyDeviceToHost, c->stream));
+        NB2_CUDA(c, cudaMemcpyAsync(b->h_status.data(), S.status, sizeof(int) * b->ninst,
+                                    cudaMemcpyDeviceToHost, c->stream));
+        NB2_CUDA(c, cudaStreamSynchronize(c->stream));
+        NB2_CUDA(c, cudaGetLastError());
+        return NB2_OK;
+    };
+    if (b->plan) {
+        NB2_TRY(read_done());
+        std::vector<int> active(b->ninst);
+        for (int i = 0; i < b->ninst; ++i) active[i] = !b->h_done[i];
+        if (any(active)) {
+            const GroupScalars G{S.thr,   S.absnew, S.beta,   S.rr,   S.rrcap,
+                                 S.iters, S.done,   S.status, S.maxit};
+            if (mode == kModeK64)
+                NB2_TRY((group_cg<double, double>(c, b->plan, G, active, c->cg_x, c->cg_r, c->cg_p,
+                                                  c->cg_q, c->cg_inv, nullptr)));
+            else
+                NB2_TRY((group_cg<float, double>(c, b->plan, G, active, c->cg_x, c->cg_r, c->cg_p,
+                                                 c->cg_q, c->cg_inv, b->dcomp)));
+            NB2_TRY(read_done());
+            for (int v : b->h_done)
+                if (!v) {
+                    c->error = "batched PCG did not stop within its iteration limit";
+                    return NB2_E_TIMEOUT;
+                }
+        }
+        return read_results();
+    }
     const int nb = b->nchunks;
     const auto spmv64 = spmv_variant<double, double>(b->lanes);
     const auto spmv3264 = spmv_variant<float, double>(b->lanes);
@@ -669,9 +717,7 @@ int batch_pcg_iterate(nb2_ctx* c, BatchState* b, int mode, int most, bool graphs
     const bool use_graph = graphs && g != nullptr;
     int guard = 0;
     for (;;) {
-        NB2_CUDA(c, cudaMemcpyAsync(b->h_done.data(), S.done, sizeof(int) * b->ninst,
-                                    cudaMemcpyDeviceToHost, c->stream));
-        NB2_CUDA(c, cudaStreamSynchronize(c->stream));
+        NB2_TRY(read_done());
         bool all = true;
         for (int v : b->h_done) all = all && v;
         if (all) break;
@@ -685,13 +731,7 @@ int batch_pcg_iterate(nb2_ctx* c, BatchState* b, int mode, int most, bool graphs
             enqueue();
         c->launches += 3 * kBatchChunk;
     }
-    NB2_CUDA(c, cudaMemcpyAsync(b->h_iters.data(), S.iters, sizeof(int) * b->ninst,
-                                cudaMemcpyDeviceToHost, c->stream));
-    NB2_CUDA(c, cudaMemcpyAsync(b->h_status.data(), S.status, sizeof(int) * b->ninst,
-                                cudaMemcpyDeviceToHost, c->stream));
-    NB2_CUDA(c, cudaStreamSynchronize(c->stream));
-    NB2_CUDA(c, cudaGetLastError());
-    return NB2_OK;
+    return read_results();
 }
 
 // the whole FP64 solve: start, iterate, x out
@@ -751,10 +791,6 @@ const char* status_message(int st) {
         case NB2_E_NEWTON_MAXIT: return "Reached Newton-Raphson iteration limit";
         default: return "";
     }
-}
-
-bool any(const std::vector<int>& v) {
-    return std::any_of(v.begin(), v.end(), [](int x) { return x != 0; });
 }
 
 struct DeviceBuffers {
@@ -984,9 +1020,11 @@ struct BatchNewton {
                 k_b_restart_cycle<<<(ninst + 255) / 256, 256, 0, c->stream>>>(ninst, b->flag_b, S);
                 c->launches++;
             }
-            k_b_p<double><<<b->nchunks, kThreads, 0, c->stream>>>(T, c->cg_p, c->cg_r, c->cg_inv,
-                                                                  S);
-            c->launches++;
+            if (!b->plan) {  // the persistent PCG forms the next direction itself
+                k_b_p<double><<<b->nchunks, kThreads, 0, c->stream>>>(T, c->cg_p, c->cg_r,
+                                                                      c->cg_inv, S);
+                c->launches++;
+            }
             NB2_CUDA(c, cudaStreamSynchronize(c->stream));  // host vectors above
         }
         for (int i = 0; i < ninst; ++i)

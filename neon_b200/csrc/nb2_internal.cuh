@@ -106,6 +106,8 @@ struct Timer {
     cudaEvent_t a = nullptr, b = nullptr;
 };
 
+struct SellPlan;  // cg_group.cuh
+
 }  // namespace nb2
 
 struct nb2_ctx {
@@ -192,6 +194,12 @@ struct nb2_ctx {
     const int* inst_on = nullptr;
     unsigned int* inst_flags = nullptr;
     int batch_rows = 0, batch_lanes = 0;  // autotuned chunk rows / lanes per block row (0: default)
+
+    // persistent PCG: the tiled copy of K and its workspace (built on first use), SM count
+    nb2::SellPlan* sell = nullptr;
+    std::vector<int> sell_offsets;  // the systems it was built for (also when it came out null)
+    int sms = 0;                    // 0 not asked yet, -1 no cooperative launch
+    int smem_optin = 0;
 
     long long launches = 0;
     std::string error;
