@@ -10,6 +10,7 @@
 
 #include "cg_group.cuh"
 #include "host_driver.hpp"
+#include "mf_cg.cuh"
 #include "nb2_internal.cuh"
 
 namespace nb2 {
@@ -240,10 +241,11 @@ int nb2_destroy(nb2_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     release_graphs(c);
     sell_release(c->sell);
+    mf_release(c->mf);
     void* ptrs[] = {c->X,      c->conn,   c->brp,    c->bcol,   c->slot,      c->K64,
                     c->K32,    c->u,      c->u_old,  c->fint,   c->fext,      c->rhs,
                     c->du,     c->inc,    c->mask,   c->Ge,     c->Ke,        c->ep,
-                    c->epbar,  c->u_tan, c->Kcsr, c->mf_d, c->mf_c, c->mf_ye, c->nadj, c->nadj_ptr, c->nadj_pl,
+                    c->epbar,  c->u_tan, c->Kcsr, c->nadj, c->nadj_ptr,
                     c->ep_old, c->epbar_old, c->sig, c->dpar,   c->detF,      c->cg_x,
                     c->cg_r,   c->cg_p,   c->cg_q,   c->cg_inv, c->cg32_x,    c->cg32_r,
                     c->cg32_p, c->cg32_q, c->cg32_inv, c->partials, c->cgs,   c->norms,
@@ -625,15 +627,6 @@ static int solve_defect_corrected(nb2_ctx* c, const double* rhs, double* out, do
                                   double* corr, double* yvec, int* iterations, int inner,
                                   bool exact);
 
-static int solve_mixed_system(nb2_ctx* c, const double* rhs, double* out, double tol,
-                              double inner_tol, int maxit, bool graphs, double* rlin,
-                              double* corr, double* yvec, int* iterations) {
-    (void)rlin;
-    (void)corr;
-    return pcg_reliable_mixed(c, rhs, out, tol, inner_tol, maxit, yvec, iterations, graphs,
-                              true);
-}
-
 static int solve_defect_corrected(nb2_ctx* c, const double* rhs, double* out, double tol,
                                   double inner_tol, int maxit, bool graphs, double* rlin,
                                   double* corr, double* yvec, int* iterations, int inner,
@@ -736,6 +729,21 @@ extern "C" int nb2_adjoint_shear_gradient(nb2_ctx* c, const double* dJdu, int32_
 // ---------------------------------------------------------------------------------------
 namespace {
 
+// Whether the assembled K fits in L2 (126 MB, with room for the vectors).  A Newton solve then runs
+// on it in one persistent launch per linear solve (cg_group.cu), also when mixed precision is asked
+// for: FP64 is the faster of the two there (37x29x32 neo-Hooke, 77 MB: 12 us per iteration against 22 in
+// FP32 matrix-free; 20^3: 7 against 18; tet4 48^3 x 6, 127 MB: 38 against 45).  Larger hex8 solves run on the matrix-free operator in
+// either precision (FP64 at 40^3, 141 MB: 32 us against 34; 48^3: 46 against 66; 64^3: 92 against 124;
+// 100^3: 219 against 450).
+static bool k_in_l2(const nb2_ctx* c) {
+    return 72.0 * (double)c->nnzb <= (c->npe == 8 ? 100e6 : 130e6);
+}
+
+// Whether an FP64 Newton solve runs on the matrix-free operator.
+static bool mf64_pays(const nb2_ctx* c) {
+    return c->npe == 8 && !c->e_inst && !k_in_l2(c) && mf64_applies(c);
+}
+
 struct DeviceTable {
     TimeTable table;
     int* dofs = nullptr;
@@ -764,8 +772,6 @@ struct Newton {
             }
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
-        for (double* p : {rlin, corr, yvec})
-            if (p) cudaFree(p);
     }
 
     int upload(const nb2_dof_table* in, int count, std::vector<DeviceTable>& out, bool weighted) {
@@ -804,16 +810,22 @@ struct Newton {
 
     unsigned grid() const { return grid_for(c->n); }
 
-    double *rlin = nullptr, *corr = nullptr, *yvec = nullptr;  // mixed defect correction
-
-    int alloc_mixed() {
-        NB2_CUDA(c, cudaMalloc(&rlin, sizeof(double) * c->n));
-        NB2_CUDA(c, cudaMalloc(&corr, sizeof(double) * c->n));
-        NB2_CUDA(c, cudaMalloc(&yvec, sizeof(double) * c->n));
-        return NB2_OK;
-    }
-
     bool mixed() const { return o.precision == NB2_MIXED; }
+
+    bool mf64 = false;       // FP64 on the matrix-free operator: no K is assembled for the solve
+    bool k_pending = false;  // ... and the resident K is not yet that of the last tangent
+
+    // Leave the last tangent assembled in K64, as the assembled path does for later calls on the
+    // context: from the stored tangent, at the displacement it belongs to (f_int is formed again
+    // by the element pass that follows).
+    int assemble_pending() {
+        if (!k_pending) return NB2_OK;
+        k_pending = false;
+        std::swap(c->u, c->u_tan);
+        const int st = launch_element_kernel(c, MODE_STIFFNESS | MODE_FORCE, NB2_FP64);
+        std::swap(c->u, c->u_tan);
+        return st;
+    }
 
     // update (+ assemble) at the context displacement; the mixed path also stores the FP64
     // tangent coefficients for its matrix-free defect residual
@@ -826,10 +838,11 @@ struct Newton {
         // point outputs, which the nodal averages of the file output read.
         int mode = MODE_CONSTITUTIVE | MODE_FORCE;
         if (assemble)
-            mode |= mixed() ? MODE_STORE : MODE_STIFFNESS;
+            mode |= mixed() || mf64 ? MODE_STORE : MODE_STIFFNESS;
         else
             mode |= MODE_STORE;
         NB2_TRY(launch_element_kernel(c, mode, NB2_FP64));
+        k_pending = mf64 && assemble;
         t_elem += time_end();
         return read_status(c);
     }
@@ -867,7 +880,10 @@ struct Newton {
             c->launches++;
         }
         double* tmp = c->cg_q;  // free until the solve
-        if (mixed())
+        if (mf64 || (mixed() && mf64_applies(c))) {
+            NB2_TRY(mf_setup(c, false, true));
+            NB2_TRY(mf_apply64(c, c->inc, tmp));
+        } else if (mixed())
             NB2_TRY(launch_apply(c, c->inc, tmp));  // FP64 tangent, matrix-free
         else
             bsr_spmv_fp64(c, c->inc, tmp, false);
@@ -889,13 +905,12 @@ struct Newton {
         }
     }
 
-    // Mixed precision: FP64 defect correction around FP32 inner PCG solves.  The defect
-    // rlin = rhs - K du uses the FP64 tangent (matrix-free), so du converges to the solution of
-    // the same FP64 system as the FP64 path, to the same relative tolerance.
+    // Mixed precision: FP32 iterations under FP64 residual replacements, so du converges to the
+    // solution of the same FP64 system as the FP64 path, to the same relative tolerance.
     int solve_mixed(int* iterations) {
-        return solve_mixed_system(c, c->rhs, c->du, o.cg_tolerance, o.mixed_inner_tolerance,
-                                  o.cg_maximum_iterations, o.use_graphs != 0, rlin, corr, yvec,
-                                  iterations);
+        return pcg_reliable_mixed(c, c->rhs, c->du, o.cg_tolerance, o.mixed_inner_tolerance,
+                                  o.cg_maximum_iterations, c->cg_r, iterations,
+                                  o.use_graphs != 0);
     }
 
     int solve_linear() {
@@ -905,6 +920,9 @@ struct Newton {
         int st;
         if (mixed())
             st = solve_mixed(&it);
+        else if (mf64)
+            st = pcg_mf64(c, c->rhs, c->du, o.cg_tolerance, o.cg_maximum_iterations, &it, &err,
+                          o.use_graphs != 0);
         else
             st = pcg_device_fp64(c, c->rhs, c->du, o.cg_tolerance, o.cg_maximum_iterations, true,
                                  &it, &err, o.use_graphs != 0);
@@ -945,6 +963,7 @@ struct Newton {
             log.push_back({load.step_time(), k, last_cg, displacement_norm, force_norm});
             const bool converged =
                 displacement_norm <= o.displacement_tolerance && force_norm <= o.residual_tolerance;
+            if (converged) NB2_TRY(assemble_pending());
             // mesh.update_internal_variables(u_{k+1}); the next assembly is fused into it
             st = element_pass(!converged);
             if (st) return st;
@@ -1007,15 +1026,20 @@ extern "C" int nb2_static_solve(nb2_ctx* c, const nb2_solver_options* options,
     // report starts.  The mixed path assembles no K: its PCG runs on the FP32 matrix-free
     // operator, so it needs the FP32 vectors and that operator's buffers, not K32
     NB2_TRY(ensure_split_buffers(c));
+    if (nw.o.precision == NB2_MIXED && k_in_l2(c)) {
+        SellPlan* plan = nullptr;
+        NB2_TRY(sell_plan(c, {0, c->N}, 8, &plan));
+        if (plan) nw.o.precision = NB2_FP64;
+    }
     if (nw.o.precision == NB2_MIXED) {
         NB2_TRY(ensure_cg32(c));
-        NB2_TRY(ensure_mf(c));
-        NB2_TRY(nw.alloc_mixed());
+        NB2_TRY(ensure_mf(c, true, true));
         if (!(nw.o.mixed_inner_tolerance > 0)) nw.o.mixed_inner_tolerance = 1e-4;
     } else {
         NB2_TRY(ensure_k64(c));
+        nw.mf64 = mf64_pays(c) && ensure_mf(c, false, true) == NB2_OK;
         // the second K buffer the element passes zero in the background
-        if (!c->e_inst) NB2_TRY(ensure_k64_alt(c));
+        if (!c->e_inst && !nw.mf64) NB2_TRY(ensure_k64_alt(c));
     }
     // the element colouring of the Newton driver's (bit-reproducible) hex8 element passes
     if (c->npe == 8 && !c->e_inst) NB2_TRY(ensure_colouring(c));
@@ -1036,6 +1060,7 @@ extern "C" int nb2_static_solve(nb2_ctx* c, const nb2_solver_options* options,
     c->error.clear();
     c->newton_scatter = true;  // bit-reproducible Newton: coloured element passes
     int st = nw.solve();
+    if (nw.k_pending && st != NB2_E_CUDA) nw.assemble_pending();  // a solve that failed
     c->newton_scatter = false;
     if (u_out) {
         cudaMemcpyAsync(u_out, c->u, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream);

@@ -37,6 +37,7 @@
 #include <cmath>
 #include <utility>
 
+#include "mf_point.cuh"
 #include "nb2_internal.cuh"
 
 namespace nb2 {
@@ -45,8 +46,6 @@ __constant__ double c_dN_hex8[8 * 8 * 3];
 __constant__ double c_w_hex8[8];
 __constant__ double c_hex8_g;  // 1/sqrt(3) as the host computed it for c_dN_hex8
 __constant__ double c_dN_tet4[4 * 3];
-__constant__ float c_dNf_hex8[8 * 8 * 3];  // FP32 copies for the matrix-free FP32 operator
-__constant__ float c_dNf_tet4[4 * 3];
 // unit-sphere rules of the microsphere models, side by side: BO21 at 0, BO33 at 21
 __constant__ double c_sphere_r[(21 + 33) * 3];
 __constant__ double c_sphere_w[21 + 33];
@@ -486,20 +485,6 @@ __device__ __forceinline__ void aniso_block(const DaT* Da, const Real* La, const
         acc[0 * 3 + k] += La[0] * Z[0][k] + La[2] * Z[4][k] + La[1] * Z[5][k];
         acc[1 * 3 + k] += La[1] * Z[1][k] + La[2] * Z[3][k] + La[0] * Z[5][k];
         acc[2 * 3 + k] += La[2] * Z[2][k] + La[1] * Z[3][k] + La[0] * Z[4][k];
-    }
-}
-
-// sigma_a = Da eps with eps the engineering strain of the gradient G (row-major 3x3); returns
-// the symmetric stress in kinetic Voigt order
-template <typename Real, typename DaT>
-__device__ __forceinline__ void aniso_stress(const DaT* Da, const Real* G, Real* sa) {
-    const Real eps[6] = {G[0], G[4], G[8], G[5] + G[7], G[2] + G[6], G[1] + G[3]};
-#pragma unroll
-    for (int v = 0; v < 6; ++v) {
-        Real t = (Real)0;
-#pragma unroll
-        for (int w = 0; w < 6; ++w) t += (Real)Da[sym6(v, w)] * eps[w];
-        sa[v] = t;
     }
 }
 
@@ -1177,11 +1162,6 @@ static int upload_tables(nb2_ctx* c) {
     NB2_CUDA(c, cudaMemcpyToSymbol(c_dN_tet4, dNt, sizeof dNt));
     NB2_CUDA(c, cudaMemcpyToSymbol(c_sphere_r, rr, sizeof rr));
     NB2_CUDA(c, cudaMemcpyToSymbol(c_sphere_w, sw, sizeof sw));
-    float dNf[8 * 8 * 3], dNtf[12];
-    for (int i = 0; i < 8 * 8 * 3; ++i) dNf[i] = (float)dN[i];
-    for (int i = 0; i < 12; ++i) dNtf[i] = (float)dNt[i];
-    NB2_CUDA(c, cudaMemcpyToSymbol(c_dNf_hex8, dNf, sizeof dNf));
-    NB2_CUDA(c, cudaMemcpyToSymbol(c_dNf_tet4, dNtf, sizeof dNtf));
     g_tables_ready = true;
     return NB2_OK;
 }
@@ -1310,64 +1290,52 @@ int launch_element_stiffness(nb2_ctx* c, long long e, double* Ke_dev) {
     return NB2_OK;
 }
 
-template <int NPE, int MODEL>
-static void mf_setup_t(nb2_ctx* c, const ElementArgs& A) {
+template <int NPE, int MODEL, typename R>
+static void mf_setup_t(nb2_ctx* c, const ElementArgs& A, float* md,
+                       R* mc, double* de) {
     constexpr int EPC = Topo<NPE>::EPC, G = Topo<NPE>::G;
     const unsigned grid = (unsigned)((c->E + EPC - 1) / EPC);
-    k_mf_setup<NPE, MODEL><<<grid, EPC * G, 0, c->stream>>>(A, c->mf_d, c->mf_c, c->mf_ye);
+    k_mf_setup<NPE, MODEL, R><<<grid, EPC * G, 0, c->stream>>>(A, md, mc, de);
     c->launches++;
 }
 
-// FP32 matrix-free data of the tangent stored by the last MODE_STORE pass; the element
-// contributions to diag(K) are left in mf_ye for the gather that forms the Jacobi inverse
-int launch_mf_setup(nb2_ctx* c) {
-    int st = upload_tables(c);
-    if (st) return st;
-    if (!c->dpar || !c->u_tan || !c->mf_d) return NB2_E_INPUT;
+template <int NPE, typename R>
+static int mf_setup_model(nb2_ctx* c, float* md, R* mc,
+                          double* de) {
     ElementArgs A = make_args(c);
     A.u = c->u_tan;
-    const bool hex = c->npe == 8;
     switch (c->mat.model) {
-        case MODEL_LE: hex ? mf_setup_t<8, MODEL_LE>(c, A) : mf_setup_t<4, MODEL_LE>(c, A); break;
-        case MODEL_NH: hex ? mf_setup_t<8, MODEL_NH>(c, A) : mf_setup_t<4, MODEL_NH>(c, A); break;
-        case MODEL_J2: hex ? mf_setup_t<8, MODEL_J2>(c, A) : mf_setup_t<4, MODEL_J2>(c, A); break;
-        case MODEL_ML: hex ? mf_setup_t<8, MODEL_ML>(c, A) : mf_setup_t<4, MODEL_ML>(c, A); break;
-        case MODEL_MN: hex ? mf_setup_t<8, MODEL_MN>(c, A) : mf_setup_t<4, MODEL_MN>(c, A); break;
-        default: hex ? mf_setup_t<8, MODEL_MS>(c, A) : mf_setup_t<4, MODEL_MS>(c, A); break;
+        case MODEL_LE: mf_setup_t<NPE, MODEL_LE>(c, A, md, mc, de); break;
+        case MODEL_NH: mf_setup_t<NPE, MODEL_NH>(c, A, md, mc, de); break;
+        case MODEL_J2: mf_setup_t<NPE, MODEL_J2>(c, A, md, mc, de); break;
+        case MODEL_MS: mf_setup_t<NPE, MODEL_MS>(c, A, md, mc, de); break;
+        default:
+            if constexpr (sizeof(R) == 4) {
+                if (c->mat.model == MODEL_ML)
+                    mf_setup_t<NPE, MODEL_ML>(c, A, md, mc, de);
+                else
+                    mf_setup_t<NPE, MODEL_MN>(c, A, md, mc, de);
+            } else {
+                return NB2_E_INPUT;
+            }
     }
     NB2_CUDA(c, cudaGetLastError());
     return NB2_OK;
 }
 
-int mf_coefficients(int model) {
-    switch (model) {
-        case MODEL_LE: return MfCoef<MODEL_LE>::KC;
-        case MODEL_NH: return MfCoef<MODEL_NH>::KC;
-        case MODEL_J2: return MfCoef<MODEL_J2>::KC;
-        case MODEL_ML: return MfCoef<MODEL_ML>::KC;
-        case MODEL_MN: return MfCoef<MODEL_MN>::KC;
-        default: return MfCoef<MODEL_MS>::KC;
-    }
+int launch_mf_setup32(nb2_ctx* c, float* md, float* mc,
+                      double* de) {
+    NB2_TRY(upload_tables(c));
+    if (!c->dpar || !c->u_tan) return NB2_E_INPUT;
+    return c->npe == 8 ? mf_setup_model<8>(c, md, mc, de)
+                       : mf_setup_model<4>(c, md, mc, de);
 }
 
-template <int NPE, int MODEL>
-static void apply32_t(nb2_ctx* c, const float* v, float* ye, const int* done) {
-    const unsigned grid = (unsigned)((c->E + kApply32Threads - 1) / kApply32Threads);
-    k_apply32<NPE, MODEL><<<grid, kApply32Threads, 0, c->stream>>>(
-        c->E, c->conn, c->mf_d, c->mf_c, c->nqp, (float)c->mat.bulk_modulus, v, ye, done);
-}
-
-// ye = K_e v_e per element in FP32 (graph-capturable: launches only)
-void enqueue_apply32(nb2_ctx* c, const float* v, float* ye, const int* done) {
-    const bool hex = c->npe == 8;
-    switch (c->mat.model) {
-        case MODEL_LE: hex ? apply32_t<8, MODEL_LE>(c, v, ye, done) : apply32_t<4, MODEL_LE>(c, v, ye, done); break;
-        case MODEL_NH: hex ? apply32_t<8, MODEL_NH>(c, v, ye, done) : apply32_t<4, MODEL_NH>(c, v, ye, done); break;
-        case MODEL_J2: hex ? apply32_t<8, MODEL_J2>(c, v, ye, done) : apply32_t<4, MODEL_J2>(c, v, ye, done); break;
-        case MODEL_ML: hex ? apply32_t<8, MODEL_ML>(c, v, ye, done) : apply32_t<4, MODEL_ML>(c, v, ye, done); break;
-        case MODEL_MN: hex ? apply32_t<8, MODEL_MN>(c, v, ye, done) : apply32_t<4, MODEL_MN>(c, v, ye, done); break;
-        default: hex ? apply32_t<8, MODEL_MS>(c, v, ye, done) : apply32_t<4, MODEL_MS>(c, v, ye, done); break;
-    }
+int launch_mf_setup64(nb2_ctx* c, double* mc, double* de) {
+    NB2_TRY(upload_tables(c));
+    if (!c->dpar || !c->u_tan) return NB2_E_INPUT;
+    return c->npe == 8 ? mf_setup_model<8>(c, nullptr, mc, de)
+                       : mf_setup_model<4>(c, nullptr, mc, de);
 }
 
 template <int NPE>

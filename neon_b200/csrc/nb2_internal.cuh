@@ -107,6 +107,7 @@ struct Timer {
 };
 
 struct SellPlan;  // cg_group.cuh
+struct MfPlan;    // mf_cg.cuh
 
 }  // namespace nb2
 
@@ -151,21 +152,16 @@ struct nb2_ctx {
     double* detF = nullptr;
     double* u_tan = nullptr;  // displacement of the last MODE_STORE pass (its geometry)
 
-    // FP32 matrix-free tangent (mixed-precision PCG): per-element relative coordinates, per-point
-    // coefficients, per-element products / diagonal contributions, node -> element-slot lists
-    float* mf_d = nullptr;   // [E][npe*3]
-    float* mf_c = nullptr;   // [kc][nqp]
-    float* mf_ye = nullptr;  // [npe][E][3]: one plane per local node (coalesced on both sides)
+    nb2::MfPlan* mf = nullptr;  // matrix-free tangent (built on first use)
+    // node -> element slots (post-processing, colouring)
     int* nadj_ptr = nullptr; // [N+1]
     int* nadj = nullptr;     // [E*npe] element slots e*npe + a, grouped by node
-    int* nadj_pl = nullptr;  // [E*npe] the same slots as plane positions a*E + e of mf_ye
     // colour-partitioned launches (hex8, single problem): elements grouped by colour
     int* corder = nullptr;                   // [E] elements sorted by colour
     std::vector<int> h_coff;                 // colour offsets into corder
     int colour_state = 0;  // 0 not set up, 1 ready, -1 not applicable (tet4, > 64 colours)
     int scatter = NB2_SCATTER_RED;  // element-pass launch mode (nb2_set_scatter_mode)
     bool newton_scatter = false;    // set while nb2_static_solve runs: colour-partitioned
-    cudaGraphExec_t graph_mf = nullptr;
 
     // PCG workspace (FP64 and FP32 views share nothing)
     double *cg_x = nullptr, *cg_r = nullptr, *cg_p = nullptr, *cg_q = nullptr, *cg_inv = nullptr;
@@ -246,9 +242,9 @@ int launch_apply(nb2_ctx* c, const double* v, double* y);  // y = K v, FP64 matr
 int launch_element_stiffness(nb2_ctx* c, long long e, double* Ke_dev);  // one dense K_e
 int launch_adjoint_shear(nb2_ctx* c, const double* lam, double* dJdG);
 int launch_force_jvp(nb2_ctx* c, const double* v, double* y);  // exact (d f_int/du) v
-int launch_mf_setup(nb2_ctx* c);  // FP32 matrix-free data + diagonal contributions
-int mf_coefficients(int model);   // FP32 coefficients per quadrature point
-void enqueue_apply32(nb2_ctx* c, const float* v, float* ye, const int* done);
+// matrix-free data of the last MODE_STORE pass: FP32 (md, mc) or FP64 (mc), and the element contributions to diag(K)
+int launch_mf_setup32(nb2_ctx* c, float* md, float* mc, double* de);
+int launch_mf_setup64(nb2_ctx* c, double* mc, double* de);
 void element_flop_model(const nb2_ctx* c, double* flops_per_element);
 
 // pcg.cu
@@ -261,13 +257,7 @@ int pcg_device_fp64(nb2_ctx* c, const double* b, double* x, double tol, int maxi
                     int* iterations, double* error, bool use_graphs);
 int pcg_device_fp32(nb2_ctx* c, const double* b, double* x, double tol, int maxit, int* iterations,
                     double* error, bool use_graphs);
-// mixed precision with reliable updates: FP32 iterations on K32, FP64 true residual (matrix-free
-// stored tangent) every `delta` reduction; work: n doubles
-int pcg_reliable_mixed(nb2_ctx* c, const double* b, double* x, double tol, double delta,
-                       int maxit, double* work, int* iterations, bool use_graphs,
-                       bool matrix_free);
-int ensure_mf(nb2_ctx* c);  // FP32 matrix-free buffers + node adjacency
-int mf_apply(nb2_ctx* c, const double* v, double* y);  // FP32 matrix-free K v (device FP64)
+int wait_scalars(nb2_ctx* c);  // the CG scalars into h_cgs (synchronises)
 int pcg_csr_host(int n, const int* rowptr, const int* col, const double* val, const double* b,
                  double* x, double tol, int maxit, int* iterations, double* error,
                  std::string* err);

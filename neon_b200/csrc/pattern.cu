@@ -172,33 +172,27 @@ int ensure_colouring(nb2_ctx* c) {
         c->colour_state = -1;
         return NB2_OK;
     }
-    NB2_TRY(build_node_adjacency(c));
     const int E = c->E, npe = c->npe, N = c->N;
     const long long m = (long long)E * npe;
-    std::vector<int> conn(m), ptr(N + 1), adj(m);
+    std::vector<int> conn(m);
     NB2_CUDA(c, cudaMemcpyAsync(conn.data(), c->conn, sizeof(int) * m, cudaMemcpyDeviceToHost,
                                 c->stream));
-    NB2_CUDA(c, cudaMemcpyAsync(ptr.data(), c->nadj_ptr, sizeof(int) * (N + 1),
-                                cudaMemcpyDeviceToHost, c->stream));
-    NB2_CUDA(c, cudaMemcpyAsync(adj.data(), c->nadj, sizeof(int) * m, cudaMemcpyDeviceToHost,
-                                c->stream));
     NB2_CUDA(c, cudaStreamSynchronize(c->stream));
+    // first fit: the colours taken at a node are a bit mask, so an element looks at its 8 nodes instead
+    // of the up to 64 elements around them (100^3 cells: 130-230 ms with the adjacency lists)
+    std::vector<unsigned long long> taken(N, 0ull);
     std::vector<unsigned char> col(E);
     int ncol = 0;
     for (int e = 0; e < E; ++e) {
+        const int* nd = &conn[(size_t)e * npe];
         unsigned long long used = 0ull;
-        for (int a = 0; a < npe; ++a) {
-            const int n = conn[(size_t)e * npe + a];
-            for (int p = ptr[n]; p < ptr[n + 1]; ++p) {
-                const int f = adj[p] / npe;
-                if (f < e) used |= 1ull << col[f];
-            }
-        }
+        for (int a = 0; a < npe; ++a) used |= taken[nd[a]];
         if (used == ~0ull) {
             c->colour_state = -1;
             return NB2_OK;
         }
         const int k = __builtin_ctzll(~used);
+        for (int a = 0; a < npe; ++a) taken[nd[a]] |= 1ull << k;
         col[e] = (unsigned char)k;
         ncol = std::max(ncol, k + 1);
     }

@@ -28,7 +28,9 @@
 #include <vector>
 
 #include "cg_group.cuh"
+#include "mf_cg.cuh"
 #include "nb2_internal.cuh"
+#include "reduce.cuh"
 
 namespace nb2 {
 
@@ -37,68 +39,6 @@ int reduction_blocks(const nb2_ctx*) { return 148 * 4; }
 template <typename T>
 __device__ __forceinline__ T ld_stream(const T* p) {
     return __ldcs(p);
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Block-wide sum of NV doubles into partials[blockIdx*NV + j]; returns true in the last block
-// (after which s_red holds nothing useful and the caller reduces partials itself).
-template <int NV>
-__device__ bool block_partials(double (&v)[NV], double* partials, unsigned int* counter) {
-    __shared__ double red[NV][kRedThreads / 32];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        double t = warp_sum(v[j]);
-        if (lane == 0) red[j][wid] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            double t = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[j][w];
-            partials[blockIdx.x * NV + j] = t;
-        }
-        __threadfence();
-        unsigned int ticket = atomicAdd(counter, 1u);
-        last = (ticket == gridDim.x - 1);
-    }
-    __syncthreads();
-    return last;
-}
-
-// Fixed-order sum of partials[b*NV + j] over b (called by the whole last block).
-template <int NV>
-__device__ void final_sum(const double* partials, double (&out)[NV]) {
-    __shared__ double red[NV][kRedThreads];
-    __threadfence();
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        double t = 0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-            t += *((volatile const double*)&partials[b * NV + j]);
-        red[j][threadIdx.x] = t;
-    }
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-#pragma unroll
-            for (int j = 0; j < NV; ++j) red[j][threadIdx.x] += red[j][threadIdx.x + s];
-        __syncthreads();
-    }
-#pragma unroll
-    for (int j = 0; j < NV; ++j) out[j] = red[j][0];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -237,29 +177,6 @@ __global__ void __launch_bounds__(kRedThreads) k_spmv(Bsr<V> A, const X* __restr
 template <typename V>
 constexpr int spmv_lanes() {
     return 4;
-}
-
-// 16-byte vector view of the CG vectors (float4 / double2): the update kernels move W values
-// per load and store when every vector is 16-byte aligned (device allocations are; a caller's
-// buffers may not be, then the scalar loop does all of it)
-template <typename X>
-struct Vec16;
-template <>
-struct Vec16<float> {
-    using T = float4;
-    static constexpr int W = 4;
-};
-template <>
-struct Vec16<double> {
-    using T = double2;
-    static constexpr int W = 2;
-};
-
-__device__ __forceinline__ bool aligned16(const void* a, const void* b, const void* c,
-                                          const void* d, const void* e) {
-    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
-             reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d) |
-             reinterpret_cast<uintptr_t>(e)) & 15) == 0;
 }
 
 template <typename X>
@@ -516,97 +433,9 @@ __global__ void __launch_bounds__(kRedThreads) k_bsr_apply(Bsr<V> A, const doubl
 }
 
 // ---------------------------------------------------------------------------------------
-// matrix-free FP32 operator: node-ordered gather of the per-element products
-// ---------------------------------------------------------------------------------------
-// q = sum over the node's element slots of ye (masked rows 0), p.q -> alpha (as k_spmv).  nadj
-// holds each slot's position in ye's per-node planes, so neighbouring nodes read neighbouring
-// elements' entries of one plane (coalesced)
-template <typename X>
-__global__ void __launch_bounds__(kRedThreads) k_mf_gather(int N, const int* __restrict__ nptr,
-                                                           const int* __restrict__ nadj,
-                                                           const float* __restrict__ ye,
-                                                           const X* __restrict__ p,
-                                                           X* __restrict__ q,
-                                                           const unsigned char* __restrict__ mask,
-                                                           CgScalars* s, double* partials) {
-    if (s->done) return;
-    double dot[1] = {0.0};
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
-        float y0 = 0.0f, y1 = 0.0f, y2 = 0.0f;
-        const int k1 = nptr[a + 1];
-#pragma unroll 4
-        for (int k = nptr[a]; k < k1; ++k) {
-            const long long j = 3ll * nadj[k];
-            y0 += ye[j];
-            y1 += ye[j + 1];
-            y2 += ye[j + 2];
-        }
-        const float y[3] = {y0, y1, y2};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const long long i = 3ll * a + c;
-            const X v = mask[i] ? (X)0 : (X)y[c];
-            q[i] = v;
-            dot[0] += (double)p[i] * (double)v;
-        }
-    }
-    if (block_partials<1>(dot, partials, &s->counter[0])) {
-        double tot[1];
-        final_sum<1>(partials, tot);
-        if (threadIdx.x == 0) {
-            s->pq = tot[0];
-            s->alpha = s->abs_new / tot[0];
-            if (!isfinite(s->alpha)) {
-                s->status = NB2_E_NAN;
-                s->done = 1;
-            }
-            s->counter[0] = 0;
-        }
-    }
-}
-
-// y = sum over the node's element slots of ye (no mask, no reduction)
-__global__ void k_mf_sum(int N, const int* __restrict__ nptr, const int* __restrict__ nadj,
-                         const float* __restrict__ ye, double* __restrict__ y) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= N) return;
-    float s[3] = {0.0f, 0.0f, 0.0f};
-    for (int k = nptr[a]; k < nptr[a + 1]; ++k) {
-        const long long j = 3ll * nadj[k];
-        s[0] += ye[j];
-        s[1] += ye[j + 1];
-        s[2] += ye[j + 2];
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) y[3ll * a + c] = (double)s[c];
-}
-
-__global__ void k_to_float(long long n, const double* __restrict__ a, float* __restrict__ b) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        b[i] = (float)a[i];
-}
-
-// Jacobi inverse from the per-element diagonal contributions (1 for a zero diagonal)
-__global__ void k_mf_diag(int N, const int* __restrict__ nptr, const int* __restrict__ nadj,
-                          const float* __restrict__ de, float* __restrict__ inv) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= N) return;
-    double d[3] = {0.0, 0.0, 0.0};
-    for (int k = nptr[a]; k < nptr[a + 1]; ++k) {
-        const long long j = 3ll * nadj[k];
-        d[0] += de[j];
-        d[1] += de[j + 1];
-        d[2] += de[j + 2];
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) inv[3ll * a + c] = d[c] != 0.0 ? (float)(1.0 / d[c]) : 1.0f;
-}
-
-// ---------------------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------------------
-static int wait_scalars(nb2_ctx* c) {
+int wait_scalars(nb2_ctx* c) {
     NB2_CUDA(c, cudaMemcpyAsync(c->h_cgs, c->cgs, sizeof(CgScalars), cudaMemcpyDeviceToHost,
                                 c->stream));
     NB2_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -624,13 +453,11 @@ struct CgRunner {
     X *x, *r, *p, *q, *inv;
     bool use_mask, use_graphs;
     cudaGraphExec_t* cache;
-    bool mf = false;  // FP32 matrix-free operator (V = X = float) instead of the assembled K
     int RB = 0;
     Bsr<V> A{};
 
     int setup() {
         RB = reduction_blocks(c);
-        if (mf) return NB2_OK;  // the Jacobi inverse comes from the matrix-free setup
         A = Bsr<V>{c->brp, c->bcol, vals, c->N};
         k_invdiag<V, X><<<(c->N + 255) / 256, 256, 0, c->stream>>>(A, inv);
         c->launches++;
@@ -641,17 +468,6 @@ struct CgRunner {
         const unsigned char* mask = use_mask ? c->mask : nullptr;
         const long long n = c->n;
         for (int it = 0; it < count; ++it) {
-            if constexpr (sizeof(X) == 4) {
-                if (mf) {
-                    enqueue_apply32(c, p, c->mf_ye, &c->cgs->done);
-                    k_mf_gather<X><<<RB, kRedThreads, 0, c->stream>>>(
-                        c->N, c->nadj_ptr, c->nadj_pl, c->mf_ye, p, q, c->mask, c->cgs, c->partials);
-                    k_xr<X><<<RB, kRedThreads, 0, c->stream>>>(n, x, r, p, q, inv, c->cgs,
-                                                               c->partials);
-                    k_p<X><<<RB, kRedThreads, 0, c->stream>>>(n, p, r, inv, c->cgs);
-                    continue;
-                }
-            }
             k_spmv<V, X, spmv_lanes<V>()><<<RB, kRedThreads, 0, c->stream>>>(A, p, q, mask, c->cgs,
                                                                             c->partials);
             k_xr<X><<<RB, kRedThreads, 0, c->stream>>>(n, x, r, p, q, inv, c->cgs, c->partials);
@@ -682,7 +498,7 @@ struct CgRunner {
                 NB2_CUDA(c, cudaGraphLaunch(*cache, c->stream));
             else
                 enqueue(kChunk);
-            c->launches += (mf ? 4 : 3) * kChunk;
+            c->launches += 3 * kChunk;
             NB2_TRY(wait_scalars(c));
             if (c->h_cgs->done) break;
             if (++guard > (maxit / kChunk) + 4) break;  // scalars say not done: cannot happen
@@ -727,137 +543,6 @@ static int run_bsr_cg(nb2_ctx* c, const V* vals, X* x, X* r, X* p, X* q, X* inv,
     return NB2_OK;
 }
 
-// x64[i] += xs[i]; xs[i] = 0 (fold the FP32 increment into the FP64 iterate)
-__global__ void k_fold(long long n, float* __restrict__ xs, double* __restrict__ x64) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        x64[i] += (double)xs[i];
-        xs[i] = 0.0f;
-    }
-}
-
-// r = b - y on free rows, 0 on masked rows; rs = (float) r; reduce r.r (FP64), rs.D^-1 rs
-__global__ void __launch_bounds__(kRedThreads) k_true_residual(
-    long long n, const double* __restrict__ b, const double* __restrict__ y,
-    const unsigned char* __restrict__ mask, const float* __restrict__ inv, float* __restrict__ rs,
-    CgScalars* s, double* partials, double* rr_out) {
-    double acc[2] = {0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const double ri = mask[i] ? 0.0 : b[i] - y[i];
-        const float rf = (float)ri;
-        rs[i] = rf;
-        acc[0] += ri * ri;
-        acc[1] += (double)rf * (double)(inv[i] * rf);
-    }
-    if (block_partials<2>(acc, partials, &s->counter[3])) {
-        double tot[2];
-        final_sum<2>(partials, tot);
-        if (threadIdx.x == 0) {
-            *rr_out = tot[0];
-            // continue the recurrence with the replaced residual: beta = rz_new / rz_old
-            s->beta = tot[1] / s->abs_new;
-            s->abs_new = tot[1];
-            s->rz = tot[1];
-            s->rr = tot[0];
-            // a cycle whose FP32 recurrence r.r grows to this multiple of the replaced one has
-            // diverged (CG residual norms are not monotone: a factor 1000 in the norm)
-            s->rr_cap = 1e6 * tot[0];
-            s->counter[3] = 0;
-        }
-    }
-}
-
-// Mixed-precision PCG with reliable updates (residual replacement): the iterations run in FP32
-// on K32 (FP64 dot products); whenever the FP32 residual has dropped by `delta` since the last
-// replacement (or below the final threshold), the FP32 increment is folded into the FP64 iterate
-// x, the true residual b - K x is formed in FP64 with the matrix-free tangent (the operator the
-// FP64 path assembles), and the FP32 residual is replaced by it; the search direction is kept,
-// so the Krylov space is not thrown away as a restarted defect correction does.  Stops when
-// the true residual meets ||r|| < tol ||b|| (the PCG's stop test, linear_solver.cpp:67-109).
-int pcg_reliable_mixed(nb2_ctx* c, const double* b, double* x, double tol, double delta,
-                       int maxit, double* work, int* iterations, bool use_graphs,
-                       bool matrix_free) {
-    CgRunner<float, float> cg{c,         c->K32,      c->cg32_x, c->cg32_r, c->cg32_p,
-                              c->cg32_q, c->cg32_inv, true,      use_graphs,
-                              matrix_free ? &c->graph_mf : &c->graph32};
-    cg.mf = matrix_free;
-    if (matrix_free) {
-        // FP32 operator data and the Jacobi inverse from the stored tangent
-        NB2_TRY(ensure_mf(c));
-        NB2_TRY(launch_mf_setup(c));
-        k_mf_diag<<<(c->N + 255) / 256, 256, 0, c->stream>>>(c->N, c->nadj_ptr, c->nadj_pl,
-                                                             c->mf_ye, c->cg32_inv);
-        c->launches++;
-    }
-    NB2_TRY(cg.setup());
-    const long long n = c->n;
-    const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 148 * 8);
-    NB2_CUDA(c, cudaMemsetAsync(x, 0, sizeof(double) * n, c->stream));
-    // the first pause comes after a delta reduction of ||b|| (threshold max(tol, delta)^2 b.b)
-    const double t0 = std::max(tol, delta);
-    k_init<float><<<cg.RB, kRedThreads, 0, c->stream>>>(n, b, cg.x, cg.r, cg.p, cg.inv, c->cgs,
-                                                        c->partials, t0);
-    c->launches++;
-    NB2_CUDA(c, cudaMemcpyAsync(&c->cgs->max_iterations, &maxit, sizeof(int),
-                                cudaMemcpyHostToDevice, c->stream));
-    NB2_TRY(wait_scalars(c));
-    const double b2 = c->h_cgs->rhs_norm2;
-    const double thr = std::max(tol * tol * b2, 2.2250738585072014e-308);
-    *iterations = 0;
-    if (b2 == 0.0) return NB2_OK;
-    double* rr_dev = c->norms + 6;
-    int resets = 0;
-    for (int update = 0;; ++update) {
-        if (!c->h_cgs->done) NB2_TRY(cg.run(maxit));
-        const CgScalars h = *c->h_cgs;
-        *iterations = h.iterations;
-        // a diverged cycle (its kept search direction no longer fits the replaced residual,
-        // near the FP32 operator's accuracy floor): replace the residual again and restart the
-        // cycle with p = D^-1 r, at most three times per solve
-        const bool fresh = h.status == NB2_E_CG_BREAKDOWN && resets < 3;
-        if (fresh) ++resets;
-        if (h.status && h.status != NB2_E_CG_MAXIT && !fresh) return h.status;
-        // reliable update: x += xs; r = b - K x in FP64
-        k_fold<<<grid, 256, 0, c->stream>>>(n, cg.x, x);
-        NB2_TRY(launch_apply(c, x, work));
-        k_true_residual<<<cg.RB, kRedThreads, 0, c->stream>>>(n, b, work, c->mask, cg.inv, cg.r,
-                                                              c->cgs, c->partials, rr_dev);
-        c->launches += 2;
-        double rr = 0;
-        NB2_CUDA(c, cudaMemcpyAsync(&rr, rr_dev, sizeof(double), cudaMemcpyDeviceToHost,
-                                    c->stream));
-        NB2_CUDA(c, cudaStreamSynchronize(c->stream));
-        if (std::getenv("NB2_DEBUG"))
-            std::fprintf(stderr, "[nb2] reliable update %d: its %d true |r|^2 %.6e thr %.6e\n",
-                         update, h.iterations, rr, thr);
-        if (!std::isfinite(rr)) return NB2_E_NAN;
-        if (rr < thr) return NB2_OK;
-        if (h.status == NB2_E_CG_MAXIT || h.iterations >= maxit || update > 1000)
-            return NB2_E_CG_MAXIT;
-        // continue: p = D^-1 r + beta p with the replaced residual, next pause after delta
-        const double next = std::max(thr, delta * delta * rr);
-        CgScalars upd = h;
-        upd.threshold = next;
-        upd.done = 0;
-        upd.status = 0;
-        NB2_CUDA(c, cudaMemcpyAsync(&c->cgs->threshold, &upd.threshold, sizeof(double),
-                                    cudaMemcpyHostToDevice, c->stream));
-        NB2_CUDA(c, cudaMemcpyAsync(&c->cgs->done, &upd.done, sizeof(int), cudaMemcpyHostToDevice,
-                                    c->stream));
-        NB2_CUDA(c, cudaMemcpyAsync(&c->cgs->status, &upd.status, sizeof(int),
-                                    cudaMemcpyHostToDevice, c->stream));
-        if (fresh) {
-            static const double zero = 0.0;
-            NB2_CUDA(c, cudaMemcpyAsync(&c->cgs->beta, &zero, sizeof(double),
-                                        cudaMemcpyHostToDevice, c->stream));
-        }
-        k_p<float><<<cg.RB, kRedThreads, 0, c->stream>>>(n, cg.p, cg.r, cg.inv, c->cgs);
-        c->launches++;
-        NB2_TRY(wait_scalars(c));
-    }
-}
-
 int pcg_device_fp64(nb2_ctx* c, const double* b, double* x, double tol, int maxit, bool use_mask,
                     int* iterations, double* error, bool use_graphs) {
     return run_bsr_cg<double, double>(c, c->K64, c->cg_x, c->cg_r, c->cg_p, c->cg_q, c->cg_inv, b,
@@ -878,49 +563,12 @@ void release_graphs(nb2_ctx* c) {
         g = nullptr;
     }
     if (c->graph32) cudaGraphExecDestroy(c->graph32);
-    if (c->graph_mf) cudaGraphExecDestroy(c->graph_mf);
-    c->graph32 = c->graph_mf = nullptr;
-}
-
-// y = K v with the FP32 matrix-free operator (v, y device FP64; y unmasked)
-int mf_apply(nb2_ctx* c, const double* v, double* y) {
-    NB2_TRY(ensure_k32(c));
-    NB2_TRY(ensure_mf(c));
-    NB2_TRY(launch_mf_setup(c));
-    const long long n = c->n;
-    k_to_float<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, c->stream>>>(
-        n, v, c->cg32_p);
-    enqueue_apply32(c, c->cg32_p, c->mf_ye, nullptr);
-    k_mf_sum<<<(c->N + 255) / 256, 256, 0, c->stream>>>(c->N, c->nadj_ptr, c->nadj_pl, c->mf_ye, y);
-    c->launches += 3;
-    NB2_CUDA(c, cudaGetLastError());
-    return NB2_OK;
-}
-
-// slot e*npe + a of the node adjacency -> its position a*E + e in the per-node planes of mf_ye
-__global__ void k_plane_slots(long long m, int npe, int E, const int* __restrict__ nadj,
-                              int* __restrict__ nadj_pl) {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m) return;
-    const int sl = nadj[k];
-    nadj_pl[k] = (sl % npe) * E + sl / npe;
-}
-
-int ensure_mf(nb2_ctx* c) {
-    if (c->mf_d) return NB2_OK;
-    const long long ev = (long long)c->E * c->npe * 3;
-    NB2_CUDA(c, cudaMalloc(&c->mf_d, sizeof(float) * ev));
-    NB2_CUDA(c, cudaMalloc(&c->mf_ye, sizeof(float) * ev));
-    NB2_CUDA(c, cudaMalloc(&c->mf_c, sizeof(float) * (long long)mf_coefficients(c->mat.model) *
-                                         c->nqp));
-    NB2_TRY(build_node_adjacency(c));
-    const long long m = (long long)c->E * c->npe;
-    NB2_CUDA(c, cudaMalloc(&c->nadj_pl, sizeof(int) * m));
-    k_plane_slots<<<(unsigned)((m + 255) / 256), 256, 0, c->stream>>>(m, c->npe, c->E, c->nadj,
-                                                                       c->nadj_pl);
-    c->launches++;
-    NB2_CUDA(c, cudaGetLastError());
-    return NB2_OK;
+    c->graph32 = nullptr;
+    if (c->mf) {
+        if (c->mf->graph32) cudaGraphExecDestroy(c->mf->graph32);
+        if (c->mf->graph64) cudaGraphExecDestroy(c->mf->graph64);
+        c->mf->graph32 = c->mf->graph64 = nullptr;
+    }
 }
 
 void bsr_spmv_fp64(nb2_ctx* c, const double* x, double* y, bool use_mask) {
