@@ -498,16 +498,20 @@ int nb2_pcg_solve(int32_t n, const int32_t* rowptr, const int32_t* col, const do
                   const double* b, double* x, double tol, int32_t maxit, int32_t* iterations,
                   double* error) {
     if (n <= 0 || !rowptr || !col || !values || !b || !x || maxit <= 0) return NB2_E_INPUT;
-    // the device kernels index x[col[k]] and rows rowptr[i]..rowptr[i+1]: validate first
+    // the device kernels index x[col[k]] and rows rowptr[i]..rowptr[i+1]: validated first, the columns
+    // on the device
+    // (here only if the device could not be asked)
     if (rowptr[0] != 0) return NB2_E_INPUT;
     for (int i = 0; i < n; ++i)
         if (rowptr[i + 1] < rowptr[i]) return NB2_E_INPUT;
-    for (long long k = 0; k < rowptr[n]; ++k)
-        if (col[k] < 0 || col[k] >= n) return NB2_E_INPUT;
     int it = 0;
     double err = 0;
     std::string msg;
     int st = pcg_csr_host(n, rowptr, col, values, b, x, tol, maxit, &it, &err, &msg);
+    if (st == NB2_E_CUDA)
+        for (long long k = 0; k < rowptr[n]; ++k)
+            if (col[k] < 0 || col[k] >= n) return NB2_E_INPUT;
+    if (st == NB2_E_INPUT) return st;
     if (iterations) *iterations = it;
     if (error) *error = err;
     if (st == NB2_OK) {

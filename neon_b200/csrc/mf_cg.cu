@@ -41,13 +41,6 @@ template <int NPE>
 constexpr int kThreads = NPE == 8 ? 64 : 256;
 constexpr int kIterations = 32;  // CG iterations per captured graph
 
-// wait for the kernels before this one (programmatic dependent launch), and let the next one start
-// its own prologue; neither orders anything else: the wait returns when they have completed
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_next() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // ---------------------------------------------------------------------------------------
 // plan
 // ---------------------------------------------------------------------------------------
@@ -617,7 +610,7 @@ __global__ void __launch_bounds__(kRedThreads, NPE == 8 && sizeof(R) == 4 ? 8 : 
     }
     if (block_partials<1>(dot, partials, &s->counter[0])) {
         double tot[1];
-        final_sum_fast<1>(partials, tot);
+        final_sum<1>(partials, tot);
         if (threadIdx.x == 0) {
             s->pq = tot[0];
             s->alpha = s->abs_new / tot[0];
@@ -683,7 +676,7 @@ __global__ void __launch_bounds__(kRedThreads) k_mf_xr(long long n, R* x, R* r, 
         xrz_one(x[i], r[i], z[node_at<R>(i)], p[node_at<R>(i)], q[i], inv[i], alpha, acc);
     if (block_partials<2>(acc, partials, &s->counter[1])) {
         double tot[2];
-        final_sum_fast<2>(partials, tot);
+        final_sum<2>(partials, tot);
         if (threadIdx.x == 0) {
             s->rr = tot[0];
             if (tot[0] < s->threshold) {
@@ -731,7 +724,7 @@ __global__ void __launch_bounds__(kRedThreads) k_mf_init(long long n, const doub
     }
     if (block_partials<3>(acc, partials, &s->counter[2])) {
         double tot[3];
-        final_sum_fast<3>(partials, tot);
+        final_sum<3>(partials, tot);
         if (threadIdx.x == 0) {
             s->rhs_norm2 = tot[0];
             s->threshold = fmax(tol * tol * tot[0], DBL_MIN);
@@ -783,7 +776,7 @@ __global__ void __launch_bounds__(kRedThreads) k_true_residual(
     }
     if (block_partials<2>(acc, partials, &s->counter[3])) {
         double tot[2];
-        final_sum_fast<2>(partials, tot);
+        final_sum<2>(partials, tot);
         if (threadIdx.x == 0) {
             // continue the recurrence with the replaced residual: beta = rz_new / rz_old
             s->beta = fresh ? 0.0 : tot[1] / s->abs_new;
@@ -823,22 +816,6 @@ __global__ void k_copy_double(long long n, const double* __restrict__ a, double*
 // ---------------------------------------------------------------------------------------
 unsigned vec_grid(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 148 * 8); }
 
-template <typename... Args>
-cudaError_t launch(bool pdl, cudaStream_t stream, unsigned grid, unsigned block, size_t smem,
-                   void (*kernel)(Args...), Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <typename R>
 MfView<R> view(const nb2_ctx* c) {
     const MfPlan* P = c->mf;
@@ -866,7 +843,7 @@ unsigned element_grid(const nb2_ctx* c) {
 
 template <int NPE, int MODEL, typename R>
 cudaError_t apply_t(nb2_ctx* c, bool pdl, const R* z, const R* p, const CgScalars* s) {
-    return launch(pdl, c->stream, element_grid(c), element_threads(c), 0, k_mf_apply<NPE, MODEL, R>,
+    return launch_early(pdl, c->stream, element_grid(c), element_threads(c), 0, k_mf_apply<NPE, MODEL, R>,
                   view<R>(c), (R)c->mat.bulk_modulus, z, p, s);
 }
 
@@ -985,7 +962,7 @@ struct MfRunner {
             cudaError_t e;
             if constexpr (sizeof(R) == 4) {
                 if (c->npe == 4) {
-                    e = launch(pdl, c->stream, gather_grid(c), (unsigned)kRedThreads, 0, k_mf_p,
+                    e = launch_early(pdl, c->stream, gather_grid(c), (unsigned)kRedThreads, 0, k_mf_p,
                                c->N, (const float*)z, p, (const CgScalars*)c->cgs);
                     if (e == cudaSuccess)
                         e = apply<R>(c, pdl, (const R*)p, (const R*)nullptr, c->cgs);
@@ -996,10 +973,10 @@ struct MfRunner {
                 e = apply<R>(c, pdl, z, p, c->cgs);  // hex8 only
             }
             if (e == cudaSuccess)
-                e = launch(pdl, c->stream, gather_grid(c), (unsigned)kRedThreads, 0,
+                e = launch_early(pdl, c->stream, gather_grid(c), (unsigned)kRedThreads, 0,
                            c->npe == 8 ? k_mf_gather<8, R> : k_mf_gather<4, R>, c->N, sums(c), ye, (const R*)z, p, q, (const unsigned char*)c->mask, c->cgs, c->partials);
             if (e == cudaSuccess)
-                e = launch(pdl, c->stream, (unsigned)RB, (unsigned)kRedThreads, 0, k_mf_xr<R>,
+                e = launch_early(pdl, c->stream, (unsigned)RB, (unsigned)kRedThreads, 0, k_mf_xr<R>,
                            (long long)c->n, x, r, z, (const R*)p, (const R*)q, (const R*)inv,
                            c->cgs, c->partials);
             if (e != cudaSuccess) return e;

@@ -1,4 +1,5 @@
-// reduce.cuh -- deterministic grid reductions and 16-byte vector views shared by the PCG kernels.
+// reduce.cuh -- deterministic grid reductions, 16-byte vector views and early launches shared by the
+// PCG kernels.
 #pragma once
 
 #include "nb2_internal.cuh"
@@ -44,27 +45,31 @@ __device__ bool block_partials(double (&v)[NV], double* partials, unsigned int* 
     return last;
 }
 
-// Fixed-order sum of partials[b*NV + j] over b (called by the whole last block).
+// Fixed-order sum of partials[b*NV + j] over b (called by the whole last block, kRedThreads threads):
+// threads, then warps, one barrier.
 template <int NV>
-__device__ void final_sum(const double* partials, double (&out)[NV]) {
-    __shared__ double red[NV][kRedThreads];
+__device__ __forceinline__ void final_sum(const double* partials, double (&out)[NV]) {
+    __shared__ double red[NV][kRedThreads / 32];
     __threadfence();
+    double t[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) t[j] = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kRedThreads)
+#pragma unroll
+        for (int j = 0; j < NV; ++j) t[j] += __ldcg(partials + b * NV + j);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-        double t = 0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-            t += *((volatile const double*)&partials[b * NV + j]);
-        red[j][threadIdx.x] = t;
+        t[j] = warp_sum(t[j]);
+        if ((threadIdx.x & 31) == 0) red[j][threadIdx.x >> 5] = t[j];
     }
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
 #pragma unroll
-            for (int j = 0; j < NV; ++j) red[j][threadIdx.x] += red[j][threadIdx.x + s];
-        __syncthreads();
+    for (int j = 0; j < NV; ++j) {
+        out[j] = 0.0;
+#pragma unroll
+        for (int w = 0; w < kRedThreads / 32; ++w) out[j] += red[j][w];
     }
-#pragma unroll
-    for (int j = 0; j < NV; ++j) out[j] = red[j][0];
 }
 
 // 16-byte vector view of the CG vectors (float4 / double2): the update kernels move W values
@@ -90,30 +95,30 @@ __device__ __forceinline__ bool aligned16(const void* a, const void* b, const vo
              reinterpret_cast<uintptr_t>(e)) & 15) == 0;
 }
 
-// The same sum in another fixed order, with one barrier: threads, then warps (kRedThreads threads).
-template <int NV>
-__device__ __forceinline__ void final_sum_fast(const double* partials, double (&out)[NV]) {
-    __shared__ double red[NV][kRedThreads / 32];
-    __threadfence();
-    double t[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) t[j] = 0.0;
-#pragma unroll 4
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += kRedThreads)
-#pragma unroll
-        for (int j = 0; j < NV; ++j) t[j] += __ldcg(partials + b * NV + j);
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        t[j] = warp_sum(t[j]);
-        if ((threadIdx.x & 31) == 0) red[j][threadIdx.x >> 5] = t[j];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        out[j] = 0.0;
-#pragma unroll
-        for (int w = 0; w < kRedThreads / 32; ++w) out[j] += red[j][w];
-    }
+// wait for the kernels before this one (programmatic dependent launch; nothing to wait for after an
+// ordinary one), and let the next one start its own prologue; neither orders anything else: the wait
+// returns when they have completed
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// launch a kernel that may start while the one before it runs (pdl); it has to call pdl_wait before
+// it touches anything that one writes
+template <typename... Args>
+cudaError_t launch_early(bool pdl, cudaStream_t stream, unsigned grid, unsigned block,
+                         size_t smem, void (*kernel)(Args...), Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace nb2
