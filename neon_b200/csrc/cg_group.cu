@@ -6,17 +6,25 @@
 // kernels per iteration (SpMV, x/r update, p update), two of them ending in a last-block
 // reduction, took 17-20 us per iteration whatever the size below 20^3 hex8 cells (27 us at
 // 37x29x32), and up to 31 iterations past convergence ran empty.  Here a group of CTAs owns a
-// system.  A CTA keeps p of every row it reads (its halo), its rows' vectors and as much of its
+// system.  A CTA keeps z of every row it reads (its halo), its rows' vectors and as much of its
 // rows of K as fit in shared memory; the rest of K streams from L2 through rings of bulk copies that
 // run ahead across the sums, since K does not change (41 bytes per cycle and SM; ordinary coalesced
-// loads, four steps in flight per warp, reached 19).  Only z = D^-1 r crosses between CTAs:
-//   1  p = z + beta p over the halo, q = K p, p.q                        -> alpha
-//   2  x += alpha p, r -= alpha q, z = D^-1 r, r.r and r.z                -> stop test, beta
-// Each line ends in a sum over the group, in which every member adds the same numbers in the same
-// order: all take the same decision and a solve is bit-reproducible.  Members exchange partial sums
-// and z as 16-byte {value, tag} pairs, written and read in one access: a reader waits for the tag
+// loads, four steps in flight per warp, reached 19).
+//
+// An iteration sums once over the group (Chronopoulos and Gear, J. Comput. Appl. Math. 25, 1989): with
+// w = K z, s = K p follows from s = w + beta s, and p.s = z.w - beta^2 (p.s of the last), so that
+//   1  z of the halo, the only vector that crosses between CTAs
+//   2  w = K z and z.w; one sum of z.w, r.r and r.z                       -> stop test, beta, alpha
+//   3  p = z + beta p, s = w + beta s, x += alpha p, r -= alpha s, z = D^-1 r
+// The textbook form sums twice (p.q, then r.r and r.z); what the second sum costs is latency, the same
+// at every size: 6.0 -> 5.0 us per iteration at 12^3 hex8 cells, 6.6 -> 5.6 at 20^3, 10.6 -> 9.4 at
+// 28^3, 11.6 -> 11.7 at 37x29x32 (two more vectors in shared memory leave less room for K), with the
+// iteration counts and the errors of before.  The first iteration of
+// a launch takes the textbook form (s = K p, p.s), because its p may carry on from an earlier launch.
+// In the sum every member adds the same numbers in the same order: all take the same decision and a
+// solve is bit-reproducible.  Members exchange partial sums and z as 16-byte {value, tag} pairs, written and read in one access: a reader waits for the tag
 // it expects, so nothing needs a fence or a separate barrier.  A z is overwritten only after the
-// next p.q sum, to which every reader contributes after its reads.  Sums go over m1 CTAs, then over
+// sum that follows it, to which every reader contributes after its reads.  Sums go over m1 CTAs, then over
 // m2 such groups (a push to each peer's own slots): 2.1 k cycles for up to 16 CTAs and 3.6 k for
 // 144, where an arrival count with release and acquire took 3.8 k and 4.8 k, and polling all
 // partials in one place 9.8 k (every SM then polls the same 37 lines).
@@ -38,7 +46,8 @@ constexpr int kGW = kGT / 32;
 constexpr int kStages = 2;           // chunks in flight per warp
 constexpr int kCopyLimit = 1 << 22;  // tries on one bulk copy (each suspends for a while)
 constexpr int kSide = 16;            // most CTAs of one level of a sum
-constexpr int kSlots = 2 * 2 * kSide * 2;  // exchange slots of a CTA
+constexpr int kValues = 3;           // values of a sum
+constexpr int kSlots = 2 * 2 * kSide * kValues;  // exchange slots of a CTA
 constexpr int kPollLimit = 1 << 22;  // polls of one tag inside an iteration (seconds)
 constexpr int kStartLimit = 1 << 26; // polls while other members still finish earlier systems
 
@@ -49,28 +58,33 @@ template <typename V>
 struct Step {
     static constexpr int VB = 32 * B * B * (int)sizeof(V);  // value bytes of a step
     static constexpr int CB = 32 * 2;                       // column bytes
-    static constexpr int CS = 4608 / VB;                    // steps of a ring chunk: 2 or 4
+    static constexpr int CS = 2;                            // steps of a ring chunk
     static constexpr int RB = CS * (VB + CB);               // bytes of a ring chunk
 };
 
-// Shared memory of a part: p and the row numbers of its halo and its tiles' first steps; the own
-// rows' x, r, D^-1 and q where they leave room for the rings; then K, or the rings and as many
-// steps of K as fit behind them.
+// Shared memory of a part: z and the row numbers of its halo and its tiles' first steps; then as many
+// of the own rows' six vectors as leave room for the rings (the others stay in global memory); then
+// K, or the rings and as many steps of K as fit behind them.
+constexpr int kVectors = 6;  // w, r, s, p, x, D^-1
 struct PartLayout {
-    bool fits, vectors;
-    int vec, ring, k, room;  // byte offsets; steps of K that are resident
+    bool fits;
+    int vectors;             // resident ones
+    int vec, bytes;          // offset of the first, bytes of each
+    int ring, k, room;       // offsets; steps of K that are resident
 };
 
 template <typename V, typename X>
 __host__ __device__ inline PartLayout part_layout(int nh, int nt, int nd, int steps, int bytes) {
     constexpr int step = Step<V>::VB + Step<V>::CB, rings = kGW * kStages * Step<V>::RB;
     const long long p = ((long long)(sizeof(X) * B + 4) * nh + 4ll * (nt + 1) + 127) / 128 * 128;
-    const long long vec = (4ll * sizeof(X) * nd + 127) / 128 * 128;
+    const long long one = ((long long)sizeof(X) * nd + 127) / 128 * 128;
     PartLayout L;
     L.fits = p + rings <= bytes;
-    L.vectors = p + vec + rings <= bytes;
+    L.vectors = kVectors;
+    while (L.vectors > 0 && p + L.vectors * one + rings > bytes) --L.vectors;
     L.vec = (int)p;
-    L.ring = (int)(L.vectors ? p + vec : p);
+    L.bytes = (int)one;
+    L.ring = (int)(p + L.vectors * one);
     const bool all = L.ring + (long long)steps * step <= bytes;
     L.k = all ? L.ring : L.ring + rings;
     L.room = all ? steps : (bytes - L.k) / step;
@@ -84,19 +98,19 @@ struct GroupArgs {
     const V* val;
     const GroupTurn* turns;
     const int* turn_ptr;
-    X *x, *r, *p, *q;
+    X *x, *r, *p, *w, *s;
     double* z;
     const X* inv;
     const float* dc;
     GroupScalars S;
-    double* slots;   // per member [2 levels][2 parities][kSide][2 values]{value, tag}
+    double* slots;   // per member [2 levels][2 parities][kSide][kValues]{value, tag}
     unsigned long long tag0;  // of this launch
     int smem_bytes;  // all of the dynamic shared memory
 };
 
 struct GroupShared {
-    double red[2][2][kGW];  // by parity: one barrier per sum orders its reuse in a group of one
-    double sum[2];
+    double red[2][4][kGW];  // by parity: one barrier per sum orders its reuse in a group of one
+    double sum[4];
     unsigned long long bar[kGW][kStages];
     int failed;
 };
@@ -119,11 +133,11 @@ __device__ __forceinline__ void tag_load(const double* a, double& v, unsigned lo
     v = __longlong_as_double(lo);
 }
 
-// One level of a sum, by one warp: lane (h, j) = (lane / 16, lane % 16) sends its value h to member
-// j's slots and waits for member j's; every lane returns the sum of value h over the n members.
-__device__ __forceinline__ double level_sum(double* to, const double* from, double v, int n,
+// One level of a sum, by one warp for two values: lane (h, j) = (lane / 16, lane % 16) sends its value
+// h to member j's slots and waits for member j's; every lane returns the sum of value h over the n
+// members.
+__device__ __forceinline__ double level_sum(double* to, const double* from, double v, bool on,
                                             unsigned long long tag, int limit, int& failed) {
-    const bool on = (threadIdx.x & 15) < n;
     if (on) tag_store(to, v, tag);
     double got = 0.0;
     unsigned long long t = tag;
@@ -141,52 +155,57 @@ __device__ __forceinline__ double level_sum(double* to, const double* from, doub
     return a;
 }
 
-// Sum of (v0, v1) over all threads of the group, the same bits in every CTA.  False when a wait
-// ran out.
+// Sum of v over all threads of the group, the same bits in every CTA; warp 0 sends the first two
+// values, warp 1 the third.  False when a wait ran out.
 __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const GroupTurn& g,
-                                          unsigned long long tag, int limit, double& v0,
-                                          double& v1) {
+                                          unsigned long long tag, int limit,
+                                          double (&v)[kValues]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int par = (int)(tag & 1);
-    double(&red)[2][kGW] = sh.red[par];
+    double(&red)[4][kGW] = sh.red[par];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-        v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < kValues; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     if (lane == 0) {
-        red[0][warp] = v0;
-        red[1][warp] = v1;
+#pragma unroll
+        for (int k = 0; k < kValues; ++k) red[k][warp] = v[k];
+        red[kValues][warp] = 0.0;
     }
     __syncthreads();
-    static_assert(kGW == kSide, "a warp's halves add the warps' sums");
-    const int h = lane >> 4, j = lane & 15;
+    static_assert(kGW == kSide && kValues == 3, "a warp's halves add the warps' sums");
+    const int j = lane & 15;
     if (g.m1 == 1) {  // alone: every warp adds the warps' sums itself
-        double a = red[h][j];
+        double a = red[lane >> 4][j], b = red[2][j];
 #pragma unroll
-        for (int o = kGW / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        v0 = __shfl_sync(0xffffffffu, a, 0);
-        v1 = __shfl_sync(0xffffffffu, a, 16);
+        for (int o = kGW / 2; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+        }
+        v[0] = __shfl_sync(0xffffffffu, a, 0);
+        v[1] = __shfl_sync(0xffffffffu, a, 16);
+        v[2] = b;
         return !sh.failed;
     }
-    if (warp == 0) {
+    if (warp < 2) {
+        const int h = 2 * warp + (lane >> 4);
         double a = red[h][j];
 #pragma unroll
         for (int o = kGW / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         const int row = g.rank / g.m1, i = g.rank - row * g.m1;
         auto slot = [&](int member, int level, int from) {
-            return slots + 2ll * (member * kSlots + ((level * 2 + par) * kSide + from) * 2 + h);
+            return slots + 2ll * (member * kSlots + ((level * 2 + par) * kSide + from) * kValues + h);
         };
-        a = level_sum(slot(row * g.m1 + j, 0, i), slot(g.rank, 0, j), a, g.m1, tag, limit,
-                      sh.failed);
+        a = level_sum(slot(row * g.m1 + j, 0, i), slot(g.rank, 0, j), a, h < kValues && j < g.m1, tag,
+                      limit, sh.failed);
         if (g.m2 > 1)
-            a = level_sum(slot(j * g.m1 + i, 1, row), slot(g.rank, 1, j), a, g.m2, tag, limit,
-                          sh.failed);
+            a = level_sum(slot(j * g.m1 + i, 1, row), slot(g.rank, 1, j), a,
+                          h < kValues && j < g.m2, tag, limit, sh.failed);
         if (j == 0) sh.sum[h] = a;
     }
     __syncthreads();
-    v0 = sh.sum[0];
-    v1 = sh.sum[1];
+#pragma unroll
+    for (int k = 0; k < kValues; ++k) v[k] = sh.sum[k];
     return !sh.failed;
 }
 
@@ -194,7 +213,7 @@ __device__ __forceinline__ unsigned smem_addr(const void* p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
 
-// one lane's share of q = K p for one step: the entry's block times its column's p
+// one lane's share of w = K z for one step: the entry's block times its column's z
 template <typename V, typename X>
 __device__ __forceinline__ void step_product(const V* v, int c, const X* p, X (&y)[B]) {
     X pn[B];
@@ -291,16 +310,20 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
         const long long d0 = (long long)B * row0;
         const int nd = B * (row1 - row0);
         const int h0 = A.halo_ptr[g.part], nh = A.halo_ptr[g.part + 1] - h0;
-        const int pown = B * A.own0[g.part];
+        const int own = A.own0[g.part], nown = row1 - row0, pown = B * own;
         const int off0 = A.tile_off[tb], nsteps = A.tile_off[te] - off0;
         const PartLayout lay = part_layout<V, X>(nh, te - tb, nd, nsteps, A.smem_bytes);
         if (!lay.fits) break;  // the plan checked every part
-        X* sp = reinterpret_cast<X*>(dyn);
+        X* sp = reinterpret_cast<X*>(dyn);  // z of the halo (p in the first iteration)
         int* shalo = reinterpret_cast<int*>(sp + (size_t)B * nh);
         int* soff = shalo + nh;
-        const bool vs = lay.vectors;
-        X* sx = reinterpret_cast<X*>(dyn + lay.vec);
-        X *sr = sx + nd, *si = sr + nd, *sq = si + nd;
+        auto vector = [&](int k, X* global) {
+            return k < lay.vectors ? reinterpret_cast<X*>(dyn + lay.vec + k * lay.bytes)
+                                   : global + d0;
+        };
+        X *vw = vector(0, A.w), *vr = vector(1, A.r), *vs = vector(2, A.s), *vp = vector(3, A.p),
+          *vx = vector(4, A.x);
+        const X* vi = vector(5, const_cast<X*>(A.inv));
         unsigned char* kbuf = dyn + lay.k;
         int tr = tb;  // tiles [tb, tr) are resident
         while (tr < te && A.tile_off[tr + 1] - off0 <= lay.room) ++tr;
@@ -337,52 +360,52 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
             for (int i = tid; i < rsteps * (S::CB / 16); i += kGT) cd[i] = cs[i];
         }
         for (int t = tb + tid; t <= te; t += kGT) soff[t - tb] = A.tile_off[t] - off0;
+        double absnew = A.S.absnew[job], beta = A.S.beta[job], rr = A.S.rr[job];
+        X bx = (X)beta;
         for (int i = tid; i < nh; i += kGT) {
             const int a = A.halo[h0 + i];
             shalo[i] = a;
+            if (i < own || i >= own + nown)
 #pragma unroll
-            for (int k = 0; k < B; ++k) sp[B * i + k] = A.p[(long long)B * a + k];
+                for (int k = 0; k < B; ++k) sp[B * i + k] = A.p[(long long)B * a + k];
         }
         for (int i = tid; i < nd; i += kGT) {
-            const X r0 = A.r[d0 + i], iv = A.inv[d0 + i];
-            if (!alone) tag_store(A.z + 2 * (d0 + i), (double)(iv * r0), tag);
-            if (vs) {
-                sx[i] = A.x[d0 + i];
-                sr[i] = r0;
-                si[i] = iv;
-            }
+            const X r0 = A.r[d0 + i], iv = A.inv[d0 + i], z0 = iv * r0;
+            if (!alone) tag_store(A.z + 2 * (d0 + i), (double)z0, tag + 1);
+            sp[pown + i] = z0 + bx * A.p[d0 + i];
+            if (lay.vectors > 1) vr[i] = r0;
+            if (lay.vectors > 4) vx[i] = A.x[d0 + i];
+            if (lay.vectors > 5) const_cast<X*>(vi)[i] = iv;
         }
-        double absnew = A.S.absnew[job], beta = A.S.beta[job], rr = A.S.rr[job];
         const double thr = A.S.thr[job], rrcap = A.S.rrcap[job];
         int iters = A.S.iters[job], status = 0;
         const int maxit = A.S.maxit[job];
-        double v0, v1;
+        double v[kValues] = {0.0, 0.0, 0.0}, pq = 0.0;
+        bool first = true;
         // the members may come from other systems: a longer wait until all are here
         int limit = kStartLimit;
         bool ok = true;
         __syncthreads();
         for (;;) {
-            // 1: p over the halo, q = K p, p.q
-            const X bx = (X)beta;
-            if (alone) {  // the halo is the system itself
-                for (int i = tid; i < nd; i += kGT) {
-                    const X zi = vs ? si[i] * sr[i] : A.inv[d0 + i] * A.r[d0 + i];
-                    sp[i] = zi + bx * sp[i];
-                }
-            } else {
-                constexpr int U = 4;
-                for (int i0 = tid; i0 < B * nh; i0 += U * kGT) {
+            // 1: z of the halo (in the first iteration p, which may carry on from an earlier launch)
+            ++tag;
+            if (!alone) {
+                constexpr int U = 6;  // loads in flight (4: +3% at 33^3, 8: +8% at 20^3)
+                const int outer = B * nh - nd;
+                for (int i0 = tid; i0 < outer; i0 += U * kGT) {
                     const double* at[U];
-                    double v[U];
+                    double zv[U];
                     unsigned long long t[U];
+                    int to[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
-                        const int i = i0 + u * kGT, j = i / B;
+                        const int o = i0 + u * kGT, i = o < pown ? o : o + nd, j = i / B;
                         t[u] = tag;
                         at[u] = nullptr;
-                        if (i < B * nh) {
+                        to[u] = i;
+                        if (o < outer) {
                             at[u] = A.z + 2 * ((long long)B * shalo[j] + (i - B * j));
-                            tag_load(at[u], v[u], t[u]);
+                            tag_load(at[u], zv[u], t[u]);
                         }
                     }
 #pragma unroll
@@ -392,15 +415,15 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                                 sh.failed = 1;
                                 break;
                             }
-                            tag_load(at[u], v[u], t[u]);
+                            tag_load(at[u], zv[u], t[u]);
                         }
-                        const int i = i0 + u * kGT;
-                        if (i < B * nh) sp[i] = (X)v[u] + bx * sp[i];
+                        if (at[u]) sp[to[u]] = first ? (X)zv[u] + bx * sp[to[u]] : (X)zv[u];
                     }
                 }
             }
             __syncthreads();
-            v0 = v1 = 0.0;
+            // 2: w = K z and z.w
+            v[0] = 0.0;
             auto diagonal = [&](int t) {
                 const int a = row0 + (t - tb) * (32 / kLpr) + ri;
                 return A.dc && a < row1 && sl < B ? (X)__ldg(A.dc + (long long)B * a + sl) : (X)0;
@@ -418,11 +441,8 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                     for (int k = 1; k < B; ++k) yi = sl == k ? y[k] : yi;
                     const X pi = sp[pown + (int)(i - d0)];
                     if (A.dc) yi += dci * pi;
-                    if (vs)
-                        sq[i - d0] = yi;
-                    else
-                        A.q[i] = yi;
-                    v0 += (double)pi * (double)yi;
+                    vw[i - d0] = yi;
+                    v[0] += (double)pi * (double)yi;
                 }
             };
             for (int t = tb + warp; t < tr; t += kGW) {
@@ -459,55 +479,59 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                 }
                 finish(t, dci, y);
             }
-            ok = group_sum(sh, slots, g, ++tag, limit, v0, v1);
+            ok = group_sum(sh, slots, g, tag, limit, v);
             limit = kPollLimit;
             if (!ok) break;
+            if (first) {
+                pq = v[0];
+            } else {
+                rr = v[1];
+                if (!isfinite(rr)) {
+                    status = NB2_E_NAN;
+                    break;
+                }
+                if (rr < thr) break;
+                if (rr > rrcap) {
+                    status = NB2_E_CG_BREAKDOWN;
+                    break;
+                }
+                beta = v[2] / absnew;
+                absnew = v[2];
+                if (++iters >= maxit) {
+                    status = NB2_E_CG_MAXIT;
+                    break;
+                }
+                pq = v[0] - beta * beta * pq;
+                bx = (X)beta;
+            }
             // Eigen's CG carries on through p.Ap <= 0 (an indefinite tangent); only a
             // non-finite step size is a failure
-            const double alpha = absnew / v0;
+            const double alpha = absnew / pq;
             if (!isfinite(alpha)) {
                 status = NB2_E_NAN;
                 break;
             }
-            // 2: x, r, z, r.r and r.z; z carries the tag of the sum that follows it
-            ++tag;
+            // 3: p, s = K p, x, r, z and the shares of r.r and r.z; z carries the tag of the sum
+            // that follows it
             const X ax = (X)alpha;
-            v0 = v1 = 0.0;
+            v[1] = v[2] = 0.0;
             for (int i = tid; i < nd; i += kGT) {
-                X rn, zi;
-                if (vs) {
-                    sx[i] += ax * sp[pown + i];
-                    rn = sr[i] - ax * sq[i];
-                    sr[i] = rn;
-                    zi = si[i] * rn;
-                } else {
-                    A.x[d0 + i] += ax * sp[pown + i];
-                    rn = A.r[d0 + i] - ax * A.q[d0 + i];
-                    A.r[d0 + i] = rn;
-                    zi = A.inv[d0 + i] * rn;
+                X pi = sp[pown + i], si = vw[i];
+                if (!first) {
+                    pi += bx * vp[i];
+                    si += bx * vs[i];
                 }
-                if (!alone) tag_store(A.z + 2 * (d0 + i), (double)zi, tag);
-                v0 += (double)rn * (double)rn;
-                v1 += (double)rn * (double)zi;
+                vp[i] = pi;
+                vs[i] = si;
+                vx[i] += ax * pi;
+                const X rn = vr[i] - ax * si, zi = vi[i] * rn;
+                vr[i] = rn;
+                sp[pown + i] = zi;
+                if (!alone) tag_store(A.z + 2 * (d0 + i), (double)zi, tag + 1);
+                v[1] += (double)rn * (double)rn;
+                v[2] += (double)rn * (double)zi;
             }
-            ok = group_sum(sh, slots, g, tag, limit, v0, v1);
-            if (!ok) break;
-            rr = v0;
-            if (!isfinite(rr)) {
-                status = NB2_E_NAN;
-                break;
-            }
-            if (rr < thr) break;
-            if (rr > rrcap) {
-                status = NB2_E_CG_BREAKDOWN;
-                break;
-            }
-            beta = v1 / absnew;
-            absnew = v1;
-            if (++iters >= maxit) {
-                status = NB2_E_CG_MAXIT;
-                break;
-            }
+            first = false;
         }
         // the copies still in flight (the rings run ahead)
         if (streams) {
@@ -520,11 +544,9 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
         if (!ok) break;
         // leave the state where the other kernels expect it
         for (int i = tid; i < nd; i += kGT) {
-            if (vs) {
-                A.x[d0 + i] = sx[i];
-                A.r[d0 + i] = sr[i];
-            }
-            A.p[d0 + i] = sp[pown + i];
+            if (lay.vectors > 1) A.r[d0 + i] = vr[i];
+            if (lay.vectors > 3) A.p[d0 + i] = first ? sp[pown + i] : vp[i];
+            if (lay.vectors > 4) A.x[d0 + i] = vx[i];
         }
         if (g.rank == 0 && tid == 0) {
             A.S.absnew[job] = absnew;
@@ -690,7 +712,7 @@ int group_shape(int n, int* m1) {
 // Cycles of an iteration of a system of t tiles on n CTAs: the sums and the exchange, and the
 // tiles, read from L2 at about 45 bytes per cycle and SM.
 double iteration_cost(int t, int n, double tile_bytes) {
-    return (n == 1 ? 600.0 : (n <= kSide ? 5500.0 : 8500.0)) + tile_bytes / 45.0 * t / n;
+    return (n == 1 ? 600.0 : (n <= kSide ? 4200.0 : 6500.0)) + tile_bytes / 45.0 * t / n;
 }
 
 // The number of CTAs of each system.  A system of up to `alone` tiles is one CTA's work; any other gets
@@ -819,7 +841,7 @@ SellPlan* sell_build(nb2_ctx* c, const int* h_rp, const std::vector<int>& offset
                      int value_bytes, const int* rp, const int* ci) {
     const int sms = device_sms(c);
     if (sms <= 0) return nullptr;
-    // p of a part's own rows alone must fit in shared memory
+    // z of a part's own rows alone must fit in shared memory
     if (offsets.size() == 2 && offsets[1] / sms > c->smem_optin / (8 * B + 4)) return nullptr;
     auto* P = new SellPlan();
     P->offsets = offsets;
@@ -830,6 +852,7 @@ SellPlan* sell_build(nb2_ctx* c, const int* h_rp, const std::vector<int>& offset
                     dev_copy(c, &P->tile_off, off) && dev_copy(c, &P->part_tile, part) &&
                     cudaMalloc(&P->z, 16 * unknowns) == cudaSuccess &&
                     cudaMemsetAsync(P->z, 0, 16 * unknowns, c->stream) == cudaSuccess &&
+                    cudaMalloc(&P->s, 8 * unknowns) == cudaSuccess &&
                     cudaMalloc(&P->turn_ptr, sizeof(int) * (sms + 1)) == cudaSuccess &&
                     sell_halo(c, P, part, rp, ci);
     if (!ok) {
@@ -944,7 +967,8 @@ int run(nb2_ctx* c, SellPlan* P, GroupScalars S, const std::vector<int>& active,
     A.r = r;
     A.z = P->z;
     A.p = p;
-    A.q = q;
+    A.w = q;
+    A.s = (X*)P->s;
     A.inv = inv;
     A.dc = dc;
     A.S = S;
@@ -965,7 +989,7 @@ void sell_release(SellPlan* P) {
     if (!P) return;
     void* ptrs[] = {P->tile_row, P->tile_end, P->tile_off, P->part_tile, P->halo_ptr,
                     P->halo,     P->own0,     P->col,      P->val[0],    P->val[1],
-                    P->z,        P->slots,    P->turns,    P->turn_ptr};
+                    P->z,        P->s,        P->slots,    P->turns,    P->turn_ptr};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete P;

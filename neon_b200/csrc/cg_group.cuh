@@ -42,6 +42,7 @@ struct SellPlan {
     unsigned short* col = nullptr;   // [steps][32]
     void* val[2] = {nullptr, nullptr};  // [steps][9][32]: double, float
     double* z = nullptr;             // the exchanged vector {value, tag}, 3 per row
+    double* s = nullptr;             // K p of parts whose vectors do not fit in shared memory
     double* slots = nullptr;
     unsigned launches = 0;           // part of every tag
     GroupTurn* turns = nullptr;      // device copy of the schedule

@@ -72,3 +72,17 @@ def test_persistent_pcg_is_bit_reproducible():
     pr = _problem("hex8", (12, 11, 10))
     sm = api.StaticMatrix(pr)
     assert np.array_equal(sm.solve(), sm.solve())
+
+
+def test_persistent_pcg_with_vectors_in_global_memory():
+    """Systems on so few CTAs each (about 500 rows a part) that their vectors do not all fit in shared
+    memory, against the same system on all of them: two solutions at CG rtol 1e-10 each, within the
+    1e-10 of the parity tests above."""
+    from neon_b200 import api
+    pr = _problem("tet4", (20, 20, 20))
+    u1 = api.StaticMatrix(pr).solve()
+    for precision in (api.FP64, api.MIXED):
+        b = api.BatchedStaticMatrix([pr] * 16, precision=precision)
+        u = b.solve()
+        for i in range(16):
+            assert rel_err(b.instance_displacement(i, u), u1) < 1e-10
