@@ -106,6 +106,34 @@ int nb2::read_status(nb2_ctx* c) {
     return NB2_E_NAN;
 }
 
+cudaError_t nb2::call_alloc(nb2_ctx* c, void** p, size_t bytes) {
+    if (!c->pool_tried) {
+        c->pool_tried = true;
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        unsigned long long keep = kPoolKeep;
+        if (cudaMemPoolCreate(&c->pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) !=
+                cudaSuccess) {
+            cudaGetLastError();
+            if (c->pool) cudaMemPoolDestroy(c->pool);
+            c->pool = nullptr;
+        }
+    }
+    bytes = std::max<size_t>(bytes, 1);
+    return c->pool ? cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream) : cudaMalloc(p, bytes);
+}
+
+void nb2::call_free(nb2_ctx* c, void* p) {
+    if (!p) return;
+    if (c->pool)
+        cudaFreeAsync(p, c->stream);
+    else
+        cudaFree(p);
+}
+
 template <typename T>
 static int dev_alloc(nb2_ctx* c, T** p, long long count) {
     NB2_CUDA(c, cudaMalloc((void**)p, sizeof(T) * (count > 0 ? count : 1)));
@@ -257,6 +285,7 @@ int nb2_destroy(nb2_ctx* c) {
     if (c->zstream) cudaStreamDestroy(c->zstream);
     if (c->h_cgs) cudaFreeHost(c->h_cgs);
     if (c->h_norms) cudaFreeHost(c->h_norms);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return NB2_OK;
@@ -708,10 +737,10 @@ extern "C" int nb2_adjoint_shear_gradient(nb2_ctx* c, const double* dJdu, int32_
     int it = 0;
     int st;
     double *rl = nullptr, *co = nullptr, *yv = nullptr, *grad = nullptr;
-    NB2_CUDA(c, cudaMalloc(&grad, sizeof(double) * c->E));
-    NB2_CUDA(c, cudaMalloc(&rl, sizeof(double) * c->n));
-    NB2_CUDA(c, cudaMalloc(&co, sizeof(double) * c->n));
-    NB2_CUDA(c, cudaMalloc(&yv, sizeof(double) * c->n));
+    NB2_CUDA(c, call_alloc(c, (void**)&grad, sizeof(double) * c->E));
+    NB2_CUDA(c, call_alloc(c, (void**)&rl, sizeof(double) * c->n));
+    NB2_CUDA(c, call_alloc(c, (void**)&co, sizeof(double) * c->n));
+    NB2_CUDA(c, call_alloc(c, (void**)&yv, sizeof(double) * c->n));
     // neon's assembled tangent is not the exact derivative of f_int: solve the exact system by
     // defect correction, the assembled K (FP64, or FP32 for the mixed adjoint) as inner solver
     // and the forward-mode product (d f_int/du) lambda as residual
@@ -723,8 +752,7 @@ extern "C" int nb2_adjoint_shear_gradient(nb2_ctx* c, const double* dJdu, int32_
         cudaMemcpyAsync(dJdG, grad, sizeof(double) * c->E, cudaMemcpyDeviceToHost, c->stream);
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) st = NB2_E_CUDA;
     }
-    for (double* p : {rl, co, yv, grad})
-        if (p) cudaFree(p);
+    for (double* p : {rl, co, yv, grad}) call_free(c, p);
     return st;
 }
 
@@ -771,8 +799,8 @@ struct Newton {
     ~Newton() {
         for (auto* v : {&dirichlet, &forces})
             for (auto& t : *v) {
-                if (t.dofs) cudaFree(t.dofs);
-                if (t.weights) cudaFree(t.weights);
+                call_free(c, t.dofs);
+                call_free(c, t.weights);
             }
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -790,11 +818,11 @@ struct Newton {
             d.table.t.assign(t.times, t.times + t.num_points);
             d.table.v.assign(t.values, t.values + t.num_points);
             d.count = t.num_dofs;
-            NB2_CUDA(c, cudaMalloc(&d.dofs, sizeof(int) * std::max(1, t.num_dofs)));
+            NB2_CUDA(c, call_alloc(c, (void**)&d.dofs, sizeof(int) * t.num_dofs));
             NB2_CUDA(c, cudaMemcpyAsync(d.dofs, t.dofs, sizeof(int) * t.num_dofs,
                                         cudaMemcpyHostToDevice, c->stream));
             if (weighted && t.weights) {
-                NB2_CUDA(c, cudaMalloc(&d.weights, sizeof(double) * std::max(1, t.num_dofs)));
+                NB2_CUDA(c, call_alloc(c, (void**)&d.weights, sizeof(double) * t.num_dofs));
                 NB2_CUDA(c, cudaMemcpyAsync(d.weights, t.weights, sizeof(double) * t.num_dofs,
                                             cudaMemcpyHostToDevice, c->stream));
             }
@@ -803,11 +831,12 @@ struct Newton {
         return NB2_OK;
     }
 
+    // Time of a phase: the events are read once the stream has been waited for anyway.
     void time_begin() { cudaEventRecord(ev0, c->stream); }
-    double time_end() {
-        cudaEventRecord(ev1, c->stream);
-        cudaEventSynchronize(ev1);
+    void time_end() { cudaEventRecord(ev1, c->stream); }
+    double elapsed() {
         float ms = 0;
+        cudaEventSynchronize(ev1);
         cudaEventElapsedTime(&ms, ev0, ev1);
         return ms * 1e-3;
     }
@@ -847,8 +876,10 @@ struct Newton {
             mode |= MODE_STORE;
         NB2_TRY(launch_element_kernel(c, mode, NB2_FP64));
         k_pending = mf64 && assemble;
-        t_elem += time_end();
-        return read_status(c);
+        time_end();
+        const int st = read_status(c);
+        t_elem += elapsed();
+        return st;
     }
 
     int compute_external_force() {
@@ -930,7 +961,7 @@ struct Newton {
         else
             st = pcg_device_fp64(c, c->rhs, c->du, o.cg_tolerance, o.cg_maximum_iterations, true,
                                  &it, &err, o.use_graphs != 0);
-        t_solve += time_end();
+        time_end();
         last_cg = it;
         cg_iterations += it;
         if (st == NB2_E_CG_MAXIT) c->error = "Conjugate gradient solver maximum iterations reached";
@@ -958,10 +989,15 @@ struct Newton {
             k_zero_masked<<<grid(), 256, 0, c->stream>>>(c->n, c->mask, c->rhs);
             c->launches++;
             st = solve_linear();
-            if (st) return st;
+            if (st) {
+                t_solve += elapsed();
+                return st;
+            }
             k_axpy<<<grid(), 256, 0, c->stream>>>(c->n, 1.0, c->du, c->u);
             c->launches++;
-            NB2_TRY(compute_norms(c));
+            const int norms = compute_norms(c);
+            t_solve += elapsed();
+            NB2_TRY(norms);
             update_relative_norms();
             ++newton_iterations;
             log.push_back({load.step_time(), k, last_cg, displacement_norm, force_norm});

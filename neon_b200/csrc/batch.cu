@@ -478,6 +478,7 @@ SpmvFn<V, X> spmv_variant(int lanes) {
 // host side: chunk tables and per-instance scalars
 // ---------------------------------------------------------------------------------------
 struct BatchState {
+    nb2_ctx* c = nullptr;
     int ninst = 0, nchunks = 0, rows = 32, lanes = 16;
     std::vector<int> h_first, h_count, h_node_off;
     int *row0 = nullptr, *row1 = nullptr, *inst = nullptr, *first = nullptr, *count = nullptr;
@@ -523,8 +524,7 @@ void batch_release(BatchState* b) {
         if (g) cudaGraphExecDestroy(g);
     void* ptrs[] = {b->row0, b->row1,    b->inst, b->first, b->count,  b->dbuf,
                     b->ibuf, b->tickets, b->part, b->norms, b->flag_a, b->flag_b, b->dcomp};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
+    for (void* p : ptrs) call_free(b->c, p);
     delete b;
 }
 
@@ -542,6 +542,7 @@ int batch_setup(nb2_ctx* c, const int* node_offsets, int ninst, int R, int lanes
             return NB2_E_INPUT;
         }
     auto* b = new BatchState();
+    b->c = c;
     b->ninst = ninst;
     b->rows = R;
     b->lanes = lanes;
@@ -558,7 +559,7 @@ int batch_setup(nb2_ctx* c, const int* node_offsets, int ninst, int R, int lanes
     }
     b->nchunks = (int)r0.size();
     auto upload = [&](int** d, const std::vector<int>& h) -> cudaError_t {
-        cudaError_t e = cudaMalloc(d, sizeof(int) * h.size());
+        cudaError_t e = call_alloc(c, (void**)d, sizeof(int) * h.size());
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(*d, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice,
                                 c->stream);
@@ -569,13 +570,13 @@ int batch_setup(nb2_ctx* c, const int* node_offsets, int ninst, int R, int lanes
     if (e == cudaSuccess) e = upload(&b->inst, in);
     if (e == cudaSuccess) e = upload(&b->first, b->h_first);
     if (e == cudaSuccess) e = upload(&b->count, b->h_count);
-    if (e == cudaSuccess) e = cudaMalloc(&b->dbuf, sizeof(double) * 8 * ninst);
-    if (e == cudaSuccess) e = cudaMalloc(&b->ibuf, sizeof(int) * 4 * ninst);
-    if (e == cudaSuccess) e = cudaMalloc(&b->tickets, sizeof(unsigned) * 4 * ninst);
-    if (e == cudaSuccess) e = cudaMalloc(&b->part, sizeof(double) * 5 * b->nchunks);
-    if (e == cudaSuccess) e = cudaMalloc(&b->norms, sizeof(double) * 5 * ninst);
-    if (e == cudaSuccess) e = cudaMalloc(&b->flag_a, sizeof(int) * ninst);
-    if (e == cudaSuccess) e = cudaMalloc(&b->flag_b, sizeof(int) * ninst);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->dbuf, sizeof(double) * 8 * ninst);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->ibuf, sizeof(int) * 4 * ninst);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->tickets, sizeof(unsigned) * 4 * ninst);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->part, sizeof(double) * 5 * b->nchunks);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->norms, sizeof(double) * 5 * ninst);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->flag_a, sizeof(int) * ninst);
+    if (e == cudaSuccess) e = call_alloc(c, (void**)&b->flag_b, sizeof(int) * ninst);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->dbuf, 0, sizeof(double) * 7 * ninst, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->ibuf, 0, sizeof(int) * 4 * ninst, c->stream);
     if (e == cudaSuccess)
@@ -629,7 +630,7 @@ int batch_pcg_start(nb2_ctx* c, BatchState* b, int mode, const double* rhs, doub
         k_b_invdiag<double, double><<<g, 256, 0, c->stream>>>(c->brp, c->bcol, c->K64, c->N,
                                                               c->cg_inv);
     else {
-        if (!b->dcomp) NB2_CUDA(c, cudaMalloc(&b->dcomp, sizeof(float) * c->n));
+        if (!b->dcomp) NB2_CUDA(c, call_alloc(c, (void**)&b->dcomp, sizeof(float) * c->n));
         k_b_compdiag<<<g, 256, 0, c->stream>>>(c->brp, c->bcol, c->K32, c->N, b->dcomp,
                                                c->cg_inv);
     }
@@ -794,10 +795,12 @@ const char* status_message(int st) {
 }
 
 struct DeviceBuffers {
+    nb2_ctx* c = nullptr;
     std::vector<void*> owned;
     template <typename T>
     int alloc(nb2_ctx* c, T** p, long long count) {
-        NB2_CUDA(c, cudaMalloc((void**)p, sizeof(T) * std::max<long long>(count, 1)));
+        this->c = c;
+        NB2_CUDA(c, call_alloc(c, (void**)p, sizeof(T) * count));
         owned.push_back(*p);
         return NB2_OK;
     }
@@ -810,7 +813,7 @@ struct DeviceBuffers {
         return NB2_OK;
     }
     ~DeviceBuffers() {
-        for (void* p : owned) cudaFree(p);
+        for (void* p : owned) call_free(c, p);
     }
 };
 
@@ -1249,7 +1252,7 @@ extern "C" int nb2_batch_autotune(nb2_ctx* c, int32_t num_instances, const int32
         if (st) break;
         Scalars S = b->scalars();
         S.timing = 1;
-        if (!f64 && cudaMalloc(&b->dcomp, sizeof(float) * c->n) == cudaSuccess)
+        if (!f64 && call_alloc(c, (void**)&b->dcomp, sizeof(float) * c->n) == cudaSuccess)
             cudaMemsetAsync(b->dcomp, 0, sizeof(float) * c->n, c->stream);  // timed like the solve's
         for (int L : lanes) {
             auto sweep = [&]() {

@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 
 #include "cg_group.cuh"
 
@@ -947,10 +948,17 @@ int run(nb2_ctx* c, SellPlan* P, GroupScalars S, const std::vector<int>& active,
         NB2_TRY(grow(c, &P->slots, &P->slots_cap, P->nslots, 16));
         NB2_CUDA(c, cudaMemsetAsync(P->slots, 0, 16ll * P->nslots, c->stream));
     }
-    NB2_CUDA(c, cudaMemcpyAsync(P->turns, P->h_turns.data(), sizeof(GroupTurn) * nturns,
-                                cudaMemcpyHostToDevice, c->stream));
-    NB2_CUDA(c, cudaMemcpyAsync(P->turn_ptr, P->h_turn_ptr.data(), sizeof(int) * (ncta + 1),
-                                cudaMemcpyHostToDevice, c->stream));
+    const size_t bytes = sizeof(GroupTurn) * nturns;
+    if (P->sent_turns.size() != P->h_turns.size() || P->sent_turn_ptr != P->h_turn_ptr ||
+        std::memcmp(P->sent_turns.data(), P->h_turns.data(), bytes) != 0) {
+        P->sent_turns.clear();
+        NB2_CUDA(c, cudaMemcpyAsync(P->turns, P->h_turns.data(), bytes,
+                                    cudaMemcpyHostToDevice, c->stream));
+        NB2_CUDA(c, cudaMemcpyAsync(P->turn_ptr, P->h_turn_ptr.data(), sizeof(int) * (ncta + 1),
+                                    cudaMemcpyHostToDevice, c->stream));
+        P->sent_turns = P->h_turns;
+        P->sent_turn_ptr = P->h_turn_ptr;
+    }
     GroupArgs<V, X> A;
     A.tile_row = P->tile_row;
     A.tile_end = P->tile_end;

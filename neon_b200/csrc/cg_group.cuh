@@ -47,8 +47,8 @@ struct SellPlan {
     unsigned launches = 0;           // part of every tag
     GroupTurn* turns = nullptr;      // device copy of the schedule
     int* turn_ptr = nullptr;
-    std::vector<GroupTurn> h_turns;
-    std::vector<int> h_turn_ptr;
+    std::vector<GroupTurn> h_turns, sent_turns;  // the schedule, and the one on the device
+    std::vector<int> h_turn_ptr, sent_turn_ptr;
     int turns_cap = 0, nslots = 0, slots_cap = 0;
 };
 

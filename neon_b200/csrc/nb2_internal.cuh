@@ -114,6 +114,8 @@ struct MfPlan;    // mf_cg.cuh
 struct nb2_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaMemPool_t pool = nullptr;  // memory of one call (call_alloc)
+    bool pool_tried = false;
     int device = 0;
     int N = 0, E = 0, npe = 0, nq = 0, nqp = 0, n = 0;
     long long nnzb = 0, nnz = 0;
@@ -209,6 +211,14 @@ int reduction_blocks(const nb2_ctx* c);
 
 // CUDA error -> context message + status
 int cuda_fail(nb2_ctx* c, cudaError_t e, const char* what);
+
+// Device memory that lives no longer than one call on the context, ordered on its stream.  It comes
+// from a pool of the context that keeps up to kPoolKeep bytes between calls and goes with it:
+// cudaMalloc and cudaFree wait for the device, which took 0.2 of the 5 ms of a 27-element Newton
+// solve, and now and then 0.1 to 0.9 s of a batched one.
+constexpr unsigned long long kPoolKeep = 64ull << 20;
+cudaError_t call_alloc(nb2_ctx* c, void** p, size_t bytes);
+void call_free(nb2_ctx* c, void* p);
 #define NB2_CUDA(ctx, call)                                     \
     do {                                                        \
         cudaError_t _e = (call);                                \
