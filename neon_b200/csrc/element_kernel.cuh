@@ -23,6 +23,9 @@
 template <int NPE, int MODEL, typename Real, int MODE>
 __global__ void __launch_bounds__(64, (MODEL == MODEL_J2) ? 8 : (model_aniso(MODEL) ? 4 : 8))
     k_element(ElementArgs A) {
+    // the next colour of a coloured pass may start: what precedes pdl_wait writes nothing that another
+    // element reads
+    if constexpr (NPE == 8 && (MODE & MODE_FORCE) != 0) pdl_next();
     using T = Topo<NPE>;
     constexpr int NQ = T::NQ, G = T::G, EPC = T::EPC, MAXB = T::MAXB;
     constexpr bool kFinite = (MODEL == MODEL_NH || MODEL == MODEL_MS || model_aniso(MODEL));
@@ -333,6 +336,7 @@ __global__ void __launch_bounds__(64, (MODEL == MODEL_J2) ? 8 : (model_aniso(MOD
     __syncthreads();
 
     if constexpr (kForce) {
+        if constexpr (NPE == 8) pdl_wait();
         if (valid) {
 #pragma unroll
             for (int j = 0; j < NG; ++j) {

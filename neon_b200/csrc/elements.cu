@@ -39,6 +39,7 @@
 
 #include "mf_point.cuh"
 #include "nb2_internal.cuh"
+#include "reduce.cuh"
 
 namespace nb2 {
 
@@ -1176,7 +1177,12 @@ static void launch_one(nb2_ctx* c, const ElementArgs& A) {
     constexpr int EPC = Topo<NPE>::EPC, G = Topo<NPE>::G;
     const unsigned grid = (launch_elements(c, A) + EPC - 1) / EPC;
     if (grid == 0) return;
-    k_element<NPE, MODEL, Real, MODE><<<grid, EPC * G, 0, c->stream>>>(A);
+    // The later colours of a coloured pass start early and compute while the one before them still
+    // scatters (programmatic dependent launch; they wait before their own scatter): a pass of a
+    // small mesh is the latency of its eight launches (27 elements: 66 -> 38 us; 20^3: 88 -> 58;
+    // 100^3: 0.84 -> 0.79 ms).  Not the first: it reads what the kernels before it wrote.
+    launch_early(A.order != nullptr && A.order != c->corder, c->stream, grid, EPC * G, 0,
+                 k_element<NPE, MODEL, Real, MODE>, A);
     c->launches++;
 }
 
