@@ -57,7 +57,8 @@ typedef enum nb2_model {
 /* Precision of the stiffness / inner linear solve. */
 typedef enum nb2_precision {
     NB2_FP64 = 0,  /* everything FP64: parity path */
-    NB2_MIXED = 1  /* FP32 tangent, SpMV and inner CG; FP64 residual, norms, dots, return map, det F */
+    NB2_MIXED = 1  /* FP32 tangent, SpMV and inner CG; FP64 residual, norms, dots, return map, det F
+                      (a single solve whose K fits in L2 runs in FP64, which is faster there) */
 } nb2_precision;
 
 typedef struct nb2_ctx nb2_ctx;

@@ -5,7 +5,9 @@
 // pass, SpMV and vector update covers all instances in a single launch.  What neon keeps per
 // problem stays per instance: the load stepping (adaptive_time_step.cpp:12-165), the Newton
 // decisions and norms (static_matrix.hpp:145-187, 353-467) and the PCG scalars
-// (linear_solver.cpp:67-109).  Rows are cut into chunks that never straddle two instances; each
+// (linear_solver.cpp:67-109).  The linear solves run in the persistent PCG (cg_group.cu), a group of
+// CTAs per instance.  Where its plan does not apply, and for the other per-instance vector work, rows
+// are cut into chunks that never straddle two instances; each
 // PCG kernel takes one chunk per CTA, writes a per-chunk partial, and the last chunk of an
 // instance to finish (a per-instance ticket) reduces that instance's partials in a fixed order:
 // deterministic segmented reductions with no spin waits.  An instance that has converged (or is
