@@ -763,10 +763,10 @@ namespace {
 
 // Whether the assembled K fits in L2 (126 MB, with room for the vectors).  A Newton solve then runs
 // on it in one persistent launch per linear solve (cg_group.cu), also when mixed precision is asked
-// for: FP64 is the faster of the two there (37x29x32 neo-Hooke, 77 MB: 12 us per iteration against 22 in
-// FP32 matrix-free; 20^3: 7 against 18; tet4 48^3 x 6, 127 MB: 38 against 45).  Larger hex8 solves run on the matrix-free operator in
-// either precision (FP64 at 40^3, 141 MB: 32 us against 34; 48^3: 46 against 66; 64^3: 92 against 124;
-// 100^3: 219 against 450).
+// for: FP64 is the faster of the two there (37x29x32 neo-Hooke, 77 MB: 12 us per iteration against
+// 22 in FP32 matrix-free; 20^3: 6 against 18; tet4 48^3 x 6, 127 MB: 38 against 45).  Larger hex8
+// solves run on the matrix-free operator in either precision (FP64 at 40^3, 141 MB: 32 us against
+// 34; 48^3: 46 against 66; 64^3: 92 against 124; 100^3: 219 against 450).
 static bool k_in_l2(const nb2_ctx* c) {
     return 72.0 * (double)c->nnzb <= (c->npe == 8 ? 100e6 : 130e6);
 }
