@@ -881,7 +881,7 @@ int allocate(nb2_ctx* c, T** p, long long count) {
 }
 
 int coefficients(int model) {
-    return model == MODEL_J2 ? 6 : (model == MODEL_LE ? 2 : (model_aniso(model) ? 8 + 21 : 8));
+    return model == MODEL_J2 ? 8 : (model == MODEL_LE ? 2 : (model_aniso(model) ? 8 + 21 : 8));
 }
 
 struct Scratch {  // freed on every way out

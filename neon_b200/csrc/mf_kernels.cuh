@@ -10,15 +10,15 @@
 //   md[c/4][e][c%4]  = (float)(x_a - x_0)_k, c = 3a + k (FP32 operator only; null for FP64)
 //   mc (MfCoef)      = s lam', s mu' | finite strain: then s sigma (6)
 //                  | Langevin / non-affine microsphere: then s Da (21, packed upper triangle)
-//                  | J2: mu' (negated at a plastic point), m = sqrt(-b) N as its 11 22 23 13 12
-//                    components (N is deviatoric, so m_33 = -m_11 - m_22).  The J2 tangent is
-//                    lam' I(x)I + 2 mu' I + b N(x)N with lam' = K - 2 mu'/3, and b < 0 at a
-//                    plastic point (b = -6 G^2 sigma_y(ebar) / (q_trial (3G + H)) for the linear
-//                    hardening return map), so b N(x)N = -m(x)m.  The point weight s = w det J
-//                    comes from the element's own FP32 geometry at apply time.  Six numbers per
-//                    point instead of nine, one at an elastic point.  (Were b ever positive, the
-//                    operator would drop that term: the FP64 residual replacements still
-//                    converge, only more slowly.)
+//                  | J2: mu', elastic; -mu' and m = sqrt(-b) N (its 11 22 23 13 12 components: N is
+//                    deviatoric, so m_33 = -m_11 - m_22), plastic.  The J2 tangent is
+//                    lam' I(x)I + 2 mu' I + b N(x)N with lam' = K - 2 mu'/3, and at a plastic point
+//                    of a hardening material b < 0 < mu', so b N(x)N = -m(x)m.  The point weight
+//                    s = w det J comes from the element's own geometry at apply time.  Six numbers
+//                    per point instead of nine, one at an elastic point.  A softening material
+//                    leaves that range (b > 0 where the yield stress of the last state is
+//                    negative, mu' < 0 where the present one is): such a point stores -infinity,
+//                    N, mu' and b.
 //   de[3a+i][e]      = element contribution to K_(3a+i, 3a+i)
 template <int NPE, int MODEL, typename R>
 __global__ void __launch_bounds__(64) k_mf_setup(ElementArgs A, float* __restrict__ md,
@@ -82,14 +82,21 @@ __global__ void __launch_bounds__(64) k_mf_setup(ElementArgs A, float* __restric
             b = A.dpar[2 * n + q];
 #pragma unroll
             for (int c = 0; c < 6; ++c) N6[c] = A.dpar[(3 + c) * n + q];
+            const R mu_r = (R)mu;
             const bool plastic = b != 0.0;
-            near[0] = plastic ? -(R)fmax(mu, 1e-30) : (R)mu;
-            const double sb = plastic ? sqrt(fmax(-b, 0.0)) : 0.0;
-            far[0 * n] = (R)(sb * N6[0]);
-            far[1 * n] = (R)(sb * N6[1]);
-            far[2 * n] = (R)(sb * N6[3]);
-            far[3 * n] = (R)(sb * N6[4]);
-            far[4 * n] = (R)(sb * N6[5]);
+            // what the short form cannot hold: a sign of its own, an infinity, NaN
+            const bool odd = plastic ? !(b < 0.0 && mu_r > (R)0 && mu_r < (R)INFINITY) : mu_r < (R)0;
+            const double f = odd ? 1.0 : (plastic ? sqrt(-b) : 0.0);
+            near[0] = odd ? -(R)INFINITY : (plastic ? -mu_r : mu_r);
+            far[0 * n] = (R)(f * N6[0]);
+            far[1 * n] = (R)(f * N6[1]);
+            far[2 * n] = (R)(f * N6[3]);
+            far[3 * n] = (R)(f * N6[4]);
+            far[4 * n] = (R)(f * N6[5]);
+            if (odd) {
+                far[5 * n] = mu_r;
+                far[6 * n] = (R)b;
+            }
         } else {
             near[0] = (R)(s * lam);
             near[1] = (R)(s * mu);

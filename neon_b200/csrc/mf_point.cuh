@@ -42,11 +42,12 @@ __device__ __forceinline__ void aniso_stress(const DaT* Da, const Real* G, Real*
 
 // Coefficients of a quadrature point: KC numbers, of which the product always reads the first NEAR;
 // those of an element's points lie together, [element][point][NEAR], and the others (J2: only a
-// plastic point has them; the anisotropic tangent) behind all of these, [coefficient][element][point].
+// plastic point has them, and the last two only one outside the hardening range; the anisotropic
+// tangent) behind all of these, [coefficient][element][point].
 template <int MODEL>
 struct MfCoef {
     static constexpr int KC =
-        (MODEL == MODEL_J2) ? 6 : ((MODEL == MODEL_LE) ? 2 : (model_aniso(MODEL) ? 8 + 21 : 8));
+        (MODEL == MODEL_J2) ? 8 : ((MODEL == MODEL_LE) ? 2 : (model_aniso(MODEL) ? 8 + 21 : 8));
     static constexpr int NEAR = (MODEL == MODEL_J2) ? 1 : ((MODEL == MODEL_LE) ? 2 : 8);
 };
 
@@ -70,9 +71,14 @@ __device__ __forceinline__ void point_flux(const R* J, const R* Gx, const R* nea
             G[i * 3 + k] = Gx[i * 3 + 0] * Ji[0 * 3 + k] + Gx[i * 3 + 1] * Ji[1 * 3 + k] +
                            Gx[i * 3 + 2] * Ji[2 * 3 + k];
     R cl, cm, c0 = (R)0, sw = (R)0;
+    [[maybe_unused]] R bs = (R)-1;
     if constexpr (kJ2) {
         c0 = near[0];
-        const R mu = (c0 < (R)0 ? -c0 : c0);
+        R mu = (c0 < (R)0 ? -c0 : c0);
+        if (c0 == -(R)INFINITY) {  // softening: mu' and b of any sign
+            mu = far[5 * st];
+            bs = far[6 * st];
+        }
         sw = det * kdet;
         cm = sw * mu;
         cl = sw * (Kb - ((R)2 / (R)3) * mu);
@@ -88,11 +94,11 @@ __device__ __forceinline__ void point_flux(const R* J, const R* Gx, const R* nea
         for (int k = 0; k < 3; ++k)
             S[i * 3 + k] = cm * (G[i * 3 + k] + G[k * 3 + i]) + (i == k ? ltr : (R)0);
     if constexpr (kJ2) {
-        if (c0 < (R)0) {  // plastic point: S -= s (m:G) m
+        if (c0 < (R)0) {  // plastic point: S -= s (m:G) m, or += s b (N:G) N
             const R m0 = far[0], m1 = far[st], m3 = far[2 * st], m4 = far[3 * st],
                     m5 = far[4 * st];
             const R m2 = -(m0 + m1);
-            const R bN = -sw * (m0 * G[0] + m1 * G[4] + m2 * G[8] + m3 * (G[5] + G[7]) +
+            const R bN = bs * sw * (m0 * G[0] + m1 * G[4] + m2 * G[8] + m3 * (G[5] + G[7]) +
                                     m4 * (G[2] + G[6]) + m5 * (G[1] + G[3]));
             // m symmetric (11 22 33 23 13 12)
             S[0] += bN * m0; S[4] += bN * m1; S[8] += bN * m2;
