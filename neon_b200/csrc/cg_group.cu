@@ -11,11 +11,16 @@
 // run ahead across the sums, since K does not change (41 bytes per cycle and SM; ordinary coalesced
 // loads, four steps in flight per warp, reached 19).
 //
-// An iteration sums once over the group (Chronopoulos and Gear, J. Comput. Appl. Math. 25, 1989): with
-// w = K z, s = K p follows from s = w + beta s, and p.s = z.w - beta^2 (p.s of the last), so that
+// An iteration sums once over the group (after Chronopoulos and Gear, J. Comput. Appl. Math. 25, 1989):
+// with w = K z, s = K p follows from s = w + beta s, and, K being symmetric,
+// p.s = z.w + 2 beta z.s' + beta^2 p'.s' with the last step's s' and p', so that
 //   1  z of the halo, the only vector that crosses between CTAs
-//   2  w = K z and z.w; one sum of z.w, r.r and r.z                       -> stop test, beta, alpha
+//   2  w = K z and z.w; one sum of z.w, r.r, r.z and z.s'                 -> stop test, beta, alpha
 //   3  p = z + beta p, s = w + beta s, x += alpha p, r -= alpha s, z = D^-1 r
+// z.s' is summed, not taken as -beta p'.s' as in that paper.  That shorter form assumes z.r' = 0 and
+// multiplies each error of p.s by beta^2: it holds while the recurrences run from their start, but a
+// launch that carries on along a kept direction (a replaced residual, a solve cut into launches) breaks
+// z.r' = 0, and ill-conditioned systems (near-incompressible, bulk / shear 1e4 and more) then stagnate.
 // The textbook form sums twice (p.q, then r.r and r.z); what the second sum costs is latency, the same
 // at every size: 6.0 -> 5.0 us per iteration at 12^3 hex8 cells, 6.6 -> 5.6 at 20^3, 10.6 -> 9.4 at
 // 28^3, 11.6 -> 11.7 at 37x29x32 (two more vectors in shared memory leave less room for K), with the
@@ -47,7 +52,7 @@ constexpr int kGW = kGT / 32;
 constexpr int kStages = 2;           // chunks in flight per warp
 constexpr int kCopyLimit = 1 << 22;  // tries on one bulk copy (each suspends for a while)
 constexpr int kSide = 16;            // most CTAs of one level of a sum
-constexpr int kValues = 3;           // values of a sum
+constexpr int kValues = 4;           // values of a sum
 constexpr int kSlots = 2 * 2 * kSide * kValues;  // exchange slots of a CTA
 constexpr int kPollLimit = 1 << 22;  // polls of one tag inside an iteration (seconds)
 constexpr int kStartLimit = 1 << 26; // polls while other members still finish earlier systems
@@ -110,8 +115,8 @@ struct GroupArgs {
 };
 
 struct GroupShared {
-    double red[2][4][kGW];  // by parity: one barrier per sum orders its reuse in a group of one
-    double sum[4];
+    double red[2][kValues][kGW];  // by parity: one barrier per sum orders its reuse in a group of one
+    double sum[kValues];
     unsigned long long bar[kGW][kStages];
     int failed;
 };
@@ -157,7 +162,7 @@ __device__ __forceinline__ double level_sum(double* to, const double* from, doub
 }
 
 // Sum of v over all threads of the group, the same bits in every CTA; warp 0 sends the first two
-// values, warp 1 the third.  False when a wait ran out.
+// values, warp 1 the others.  False when a wait ran out.
 __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const GroupTurn& g,
                                           unsigned long long tag, int limit,
                                           double (&v)[kValues]) {
@@ -171,13 +176,12 @@ __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const 
     if (lane == 0) {
 #pragma unroll
         for (int k = 0; k < kValues; ++k) red[k][warp] = v[k];
-        red[kValues][warp] = 0.0;
     }
     __syncthreads();
-    static_assert(kGW == kSide && kValues == 3, "a warp's halves add the warps' sums");
+    static_assert(kGW == kSide && kValues == 4, "a warp's halves add the warps' sums");
     const int j = lane & 15;
     if (g.m1 == 1) {  // alone: every warp adds the warps' sums itself
-        double a = red[lane >> 4][j], b = red[2][j];
+        double a = red[lane >> 4][j], b = red[2 + (lane >> 4)][j];
 #pragma unroll
         for (int o = kGW / 2; o > 0; o >>= 1) {
             a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -185,7 +189,8 @@ __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const 
         }
         v[0] = __shfl_sync(0xffffffffu, a, 0);
         v[1] = __shfl_sync(0xffffffffu, a, 16);
-        v[2] = b;
+        v[2] = __shfl_sync(0xffffffffu, b, 0);
+        v[3] = __shfl_sync(0xffffffffu, b, 16);
         return !sh.failed;
     }
     if (warp < 2) {
@@ -197,11 +202,11 @@ __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const 
         auto slot = [&](int member, int level, int from) {
             return slots + 2ll * (member * kSlots + ((level * 2 + par) * kSide + from) * kValues + h);
         };
-        a = level_sum(slot(row * g.m1 + j, 0, i), slot(g.rank, 0, j), a, h < kValues && j < g.m1, tag,
-                      limit, sh.failed);
+        a = level_sum(slot(row * g.m1 + j, 0, i), slot(g.rank, 0, j), a, j < g.m1, tag, limit,
+                      sh.failed);
         if (g.m2 > 1)
-            a = level_sum(slot(j * g.m1 + i, 1, row), slot(g.rank, 1, j), a,
-                          h < kValues && j < g.m2, tag, limit, sh.failed);
+            a = level_sum(slot(j * g.m1 + i, 1, row), slot(g.rank, 1, j), a, j < g.m2, tag, limit,
+                          sh.failed);
         if (j == 0) sh.sum[h] = a;
     }
     __syncthreads();
@@ -381,7 +386,7 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
         const double thr = A.S.thr[job], rrcap = A.S.rrcap[job];
         int iters = A.S.iters[job], status = 0;
         const int maxit = A.S.maxit[job];
-        double v[kValues] = {0.0, 0.0, 0.0}, pq = 0.0;
+        double v[kValues] = {0.0, 0.0, 0.0, 0.0}, pq = 0.0;
         bool first = true;
         // the members may come from other systems: a longer wait until all are here
         int limit = kStartLimit;
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                     status = NB2_E_CG_MAXIT;
                     break;
                 }
-                pq = v[0] - beta * beta * pq;
+                pq = v[0] + beta * (2.0 * v[3] + beta * pq);
                 bx = (X)beta;
             }
             // Eigen's CG carries on through p.Ap <= 0 (an indefinite tangent); only a
@@ -512,10 +517,10 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                 status = NB2_E_NAN;
                 break;
             }
-            // 3: p, s = K p, x, r, z and the shares of r.r and r.z; z carries the tag of the sum
-            // that follows it
+            // 3: p, s = K p, x, r, z and the shares of r.r, r.z and z.s; z carries the tag of the
+            // sum that follows it
             const X ax = (X)alpha;
-            v[1] = v[2] = 0.0;
+            v[1] = v[2] = v[3] = 0.0;
             for (int i = tid; i < nd; i += kGT) {
                 X pi = sp[pown + i], si = vw[i];
                 if (!first) {
@@ -531,6 +536,7 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                 if (!alone) tag_store(A.z + 2 * (d0 + i), (double)zi, tag + 1);
                 v[1] += (double)rn * (double)rn;
                 v[2] += (double)rn * (double)zi;
+                v[3] += (double)zi * (double)si;
             }
             first = false;
         }

@@ -1,0 +1,64 @@
+"""The persistent PCG on ill-conditioned systems: near-incompressible elasticity (bulk / shear 1e3 and 1e4)
+needs thousands of iterations, over which an error in a recurrence would grow.
+
+One Newton step from rest, so that the displacement is the prescribed increment plus the solution x of
+one linear system; b - K x is formed with the K of the element kernels, downloaded.  CG stops at 1e-10 |b|
+(a mixed solve on its FP64 residual); 2e-10 leaves as much again for rounding (1e-16 times the ratio of
+the largest intermediate residual to |b|, below 1e4 here).  Mixed-precision batches carry on along a kept
+direction after every replaced residual, and have to get there within 60000 iterations."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from neon_b200 import mesh as M
+from neon_b200 import problem as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(n, ratio):
+    mesh = M.structured_hex8(n, n, n, jitter=0.05, seed=3)
+    bcs = [{"name": "bottom", "time": [0.0, 1.0], "x": [0.0, 0.0], "y": [0.0, 0.0],
+            "z": [0.0, 0.0]},
+           {"name": "top", "time": [0.0, 1.0], "z": [0.0, 1e-3]}]
+    opts = P.Options(residual_tolerance=1e9, displacement_tolerance=1e9, linear_iterations=2,
+                     cg_tolerance=1e-10, cg_maximum_iterations=60000)
+    return P.Problem("incompressible", mesh, P.Material(P.LINEAR_ELASTIC, ratio, 1.0),
+                     P.dirichlet_boundaries(mesh, bcs), opts)
+
+
+def _residual(api, pr, u):
+    g = api.SolidMesh(pr.mesh.X, pr.mesh.conn, pr.material)
+    g.update_internal_variables(np.zeros(g.ndofs))
+    K, _ = g.assemble()
+    rp, col = g.sparsity_pattern()
+    A = sp.csr_matrix((K, col, rp), shape=(g.ndofs, g.ndofs))
+    inc, free = np.zeros(g.ndofs), np.ones(g.ndofs, bool)
+    for t in pr.dirichlet:
+        inc[t.dofs] = t.values[-1]
+        free[t.dofs] = False
+    b = -(A @ inc)
+    return np.linalg.norm((b - A @ (u - inc))[free]) / np.linalg.norm(b[free])
+
+
+@pytest.mark.parametrize("n", [3, 7, 14])  # one CTA, a group, two exchange levels
+@pytest.mark.parametrize("ratio", [1e3, 1e4])
+def test_true_residual(n, ratio):
+    from neon_b200 import api
+    pr = _problem(n, ratio)
+    sm = api.StaticMatrix(pr)
+    u = sm.solve()
+    assert len(sm.log) == 1 and sm.log[0, 2] > 100
+    assert _residual(api, pr, u) <= 2e-10
+
+
+@pytest.mark.parametrize("ratio", [1e3, 1e4])
+def test_batch_true_residual(ratio):
+    from neon_b200 import api
+    problems = [_problem(n, ratio) for n in (7, 3, 9)]
+    for precision in (api.FP64, api.MIXED):
+        b = api.BatchedStaticMatrix(problems, precision=precision, autotune=False)
+        u = b.solve()
+        for i, pr in enumerate(problems):
+            assert b.reports[i]["newton_iterations"] == 1
+            assert _residual(api, pr, b.instance_displacement(i, u)) <= 2e-10
