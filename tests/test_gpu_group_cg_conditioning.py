@@ -6,7 +6,9 @@ one linear system; b - K x is formed with the K of the element kernels, download
 (a mixed solve on its FP64 residual); 2e-10 leaves as much again for rounding (1e-16 times the ratio of
 the largest intermediate residual to |b|, below 1e4 here).  Mixed-precision batches carry on along a kept
 direction after every replaced residual; the three-kernel textbook PCG with the same replacements took the
-iterations below, and a quarter more is room for another order of sums."""
+iterations below.  They scatter from run to run with the order of the assembly's atomic additions, by 1%
+and, at 54 unknowns and 1e5, by up to a factor of 1.2 (both PCGs, 60 runs); twice the count is far from
+that, and from the seven times and more that a direction which lost its conjugacy takes at 1e4."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -65,5 +67,5 @@ def test_batch_true_residual(ratio):
         u = b.solve()
         for i, pr in enumerate(problems):
             assert b.reports[i]["newton_iterations"] == 1
-            assert b.reports[i]["cg_iterations"] <= 1.25 * TEXTBOOK[ratio][i]
+            assert b.reports[i]["cg_iterations"] <= 2 * TEXTBOOK[ratio][i]
             assert _residual(api, pr, b.instance_displacement(i, u)) <= 2e-10
