@@ -670,8 +670,9 @@ int batch_pcg_iterate(nb2_ctx* c, BatchState* b, int mode, int most, bool graphs
     if (b->plan) {
         NB2_TRY(read_done());
         std::vector<int> active(b->ninst);
-        for (int i = 0; i < b->ninst; ++i) active[i] = !b->h_done[i];
-        if (any(active)) {
+        for (;;) {
+            for (int i = 0; i < b->ninst; ++i) active[i] = !b->h_done[i];
+            if (!any(active)) break;
             const GroupScalars G{S.thr,   S.absnew, S.beta,   S.rr,   S.rrcap,
                                  S.iters, S.done,   S.status, S.maxit};
             if (mode == kModeK64)
@@ -680,12 +681,12 @@ int batch_pcg_iterate(nb2_ctx* c, BatchState* b, int mode, int most, bool graphs
             else
                 NB2_TRY((group_cg<float, double>(c, b->plan, G, active, c->cg_x, c->cg_r, c->cg_p,
                                                  c->cg_q, c->cg_inv, b->dcomp)));
+            NB2_TRY(wait_scalars(c));
             NB2_TRY(read_done());
-            for (int v : b->h_done)
-                if (!v) {
-                    c->error = "batched PCG did not stop within its iteration limit";
-                    return NB2_E_TIMEOUT;
-                }
+            if (group_failed(c)) {
+                c->error = "a wait of the batched PCG ran out";
+                return NB2_E_TIMEOUT;
+            }
         }
         return read_results();
     }

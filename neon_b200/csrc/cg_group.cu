@@ -34,8 +34,11 @@
 // 144, where an arrival count with release and acquire took 3.8 k and 4.8 k, and polling all
 // partials in one place 9.8 k (every SM then polls the same 37 lines).
 //
-// Co-residency comes from the cooperative launch; every wait has an iteration limit, after which
-// the CTA returns and leaves its system's `done` at 0.
+// Co-residency comes from the cooperative launch; every wait has a limit, after which the CTA reports
+// the launch as failed and returns, leaving its system's `done` at 0.  A CTA may have to wait for members
+// that still work on earlier systems.  So that such a wait has a bound that no legitimate work reaches,
+// a turn ends after kTurnIterations with its state stored, and the caller launches again (a launch
+// reloads K, 20 to 60 us in at least 10 ms).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -55,7 +58,10 @@ constexpr int kSide = 16;            // most CTAs of one level of a sum
 constexpr int kValues = 4;           // values of a sum
 constexpr int kSlots = 2 * 2 * kSide * kValues;  // exchange slots of a CTA
 constexpr int kPollLimit = 1 << 22;  // polls of one tag inside an iteration (seconds)
-constexpr int kStartLimit = 1 << 26; // polls while other members still finish earlier systems
+constexpr int kTurnIterations = 2048;  // a system's most iterations in one launch
+// polls (0.4 us and more each) for each turn that other members may still have to finish: seconds,
+// where 2048 iterations take up to 1 s for the largest parts
+constexpr int kStartLimit = 1 << 23;
 
 constexpr int kLpr = 4;              // lanes per row of a tile
 constexpr int B = 3;                 // block size
@@ -111,6 +117,8 @@ struct GroupArgs {
     GroupScalars S;
     double* slots;   // per member [2 levels][2 parities][kSide][kValues]{value, tag}
     unsigned long long tag0;  // of this launch
+    unsigned *failed, launch;  // *failed = launch: a wait of this launch ran out
+    int start_limit;
     int smem_bytes;  // all of the dynamic shared memory
 };
 
@@ -119,6 +127,8 @@ struct GroupShared {
     double sum[kValues];
     unsigned long long bar[kGW][kStages];
     int failed;
+    const unsigned* failed_launch;  // GroupArgs::failed, launch
+    unsigned launch;
 };
 
 // {value, tag} in one 16-byte access
@@ -139,19 +149,24 @@ __device__ __forceinline__ void tag_load(const double* a, double& v, unsigned lo
     v = __longlong_as_double(lo);
 }
 
+// whether a wait of this launch ran out somewhere; looked at now and then
+__device__ __forceinline__ bool others_failed(int polls, const unsigned* failed, unsigned launch) {
+    return (polls & 1023) == 1023 && *(const volatile unsigned*)failed == launch;
+}
+
 // One level of a sum, by one warp for two values: lane (h, j) = (lane / 16, lane % 16) sends its value
 // h to member j's slots and waits for member j's; every lane returns the sum of value h over the n
 // members.
 __device__ __forceinline__ double level_sum(double* to, const double* from, double v, bool on,
-                                            unsigned long long tag, int limit, int& failed) {
+                                            unsigned long long tag, int limit, GroupShared& sh) {
     if (on) tag_store(to, v, tag);
     double got = 0.0;
     unsigned long long t = tag;
     for (int k = 0;; ++k) {
         if (on) tag_load(from, got, t);
         if (__all_sync(0xffffffffu, t == tag)) break;
-        if (k > limit) {
-            failed = 1;
+        if (__any_sync(0xffffffffu, k > limit || others_failed(k, sh.failed_launch, sh.launch))) {
+            sh.failed = 1;
             break;
         }
     }
@@ -169,28 +184,24 @@ __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int par = (int)(tag & 1);
     double(&red)[4][kGW] = sh.red[par];
+    static_assert(kGW == kSide && kValues == 4, "the lanes' shares of the four values");
+    // a lane hands on what it does not keep: after two steps each quarter of the warp holds one value
+    // (6 exchanges instead of 20; a system on one CTA waits for them in every iteration)
+    const bool half = (lane & 16) != 0, quarter = (lane & 8) != 0;
+    const double s0 = (half ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, half ? v[0] : v[2], 16);
+    const double s1 = (half ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, half ? v[1] : v[3], 16);
+    double t = (quarter ? s1 : s0) + __shfl_xor_sync(0xffffffffu, quarter ? s0 : s1, 8);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < kValues; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < kValues; ++k) red[k][warp] = v[k];
-    }
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 7) == 0) red[lane >> 3][warp] = t;
     __syncthreads();
-    static_assert(kGW == kSide && kValues == 4, "a warp's halves add the warps' sums");
     const int j = lane & 15;
-    if (g.m1 == 1) {  // alone: every warp adds the warps' sums itself
-        double a = red[lane >> 4][j], b = red[2 + (lane >> 4)][j];
+    if (g.m1 == 1) {  // alone: every warp adds the warps' sums itself, a quarter for each value
+        double a = red[lane >> 3][lane & 7] + red[lane >> 3][8 + (lane & 7)];
 #pragma unroll
-        for (int o = kGW / 2; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
-        }
-        v[0] = __shfl_sync(0xffffffffu, a, 0);
-        v[1] = __shfl_sync(0xffffffffu, a, 16);
-        v[2] = __shfl_sync(0xffffffffu, b, 0);
-        v[3] = __shfl_sync(0xffffffffu, b, 16);
+        for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+#pragma unroll
+        for (int k = 0; k < kValues; ++k) v[k] = __shfl_sync(0xffffffffu, a, 8 * k);
         return !sh.failed;
     }
     if (warp < 2) {
@@ -203,10 +214,10 @@ __device__ __forceinline__ bool group_sum(GroupShared& sh, double* slots, const 
             return slots + 2ll * (member * kSlots + ((level * 2 + par) * kSide + from) * kValues + h);
         };
         a = level_sum(slot(row * g.m1 + j, 0, i), slot(g.rank, 0, j), a, j < g.m1, tag, limit,
-                      sh.failed);
+                      sh);
         if (g.m2 > 1)
             a = level_sum(slot(j * g.m1 + i, 1, row), slot(g.rank, 1, j), a, j < g.m2, tag, limit,
-                          sh.failed);
+                          sh);
         if (j == 0) sh.sum[h] = a;
     }
     __syncthreads();
@@ -296,7 +307,11 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
     __shared__ GroupShared sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ri = lane / kLpr, sl = lane % kLpr;
-    if (tid == 0) sh.failed = 0;
+    if (tid == 0) {
+        sh.failed = 0;
+        sh.failed_launch = A.failed;
+        sh.launch = A.launch;
+    }
     if (tid < kGW * kStages)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh.bar[0][0] + tid))
                      : "memory");
@@ -319,7 +334,10 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
         const int own = A.own0[g.part], nown = row1 - row0, pown = B * own;
         const int off0 = A.tile_off[tb], nsteps = A.tile_off[te] - off0;
         const PartLayout lay = part_layout<V, X>(nh, te - tb, nd, nsteps, A.smem_bytes);
-        if (!lay.fits) break;  // the plan checked every part
+        if (!lay.fits) {  // the plan checked every part
+            if (tid == 0) *(volatile unsigned*)A.failed = A.launch;
+            break;
+        }
         X* sp = reinterpret_cast<X*>(dyn);  // z of the halo (p in the first iteration)
         int* shalo = reinterpret_cast<int*>(sp + (size_t)B * nh);
         int* soff = shalo + nh;
@@ -385,11 +403,11 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
         }
         const double thr = A.S.thr[job], rrcap = A.S.rrcap[job];
         int iters = A.S.iters[job], status = 0;
-        const int maxit = A.S.maxit[job];
+        const int maxit = A.S.maxit[job], begun = iters;
         double v[kValues] = {0.0, 0.0, 0.0, 0.0}, pq = 0.0;
-        bool first = true;
+        bool first = true, paused = false;
         // the members may come from other systems: a longer wait until all are here
-        int limit = kStartLimit;
+        int limit = A.start_limit;
         bool ok = true;
         __syncthreads();
         for (;;) {
@@ -417,7 +435,7 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         for (int k = 0; t[u] != tag; ++k) {
-                            if (k > limit) {
+                            if (k > limit || others_failed(k, A.failed, A.launch)) {
                                 sh.failed = 1;
                                 break;
                             }
@@ -507,6 +525,10 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
                     status = NB2_E_CG_MAXIT;
                     break;
                 }
+                if (iters - begun >= kTurnIterations) {
+                    paused = true;
+                    break;
+                }
                 pq = v[0] + beta * (2.0 * v[3] + beta * pq);
                 bx = (X)beta;
             }
@@ -548,7 +570,10 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
             }
             chunks_used = ring.used;
         }
-        if (!ok) break;
+        if (!ok) {
+            if (tid == 0) *(volatile unsigned*)A.failed = A.launch;
+            break;
+        }
         // leave the state where the other kernels expect it
         for (int i = tid; i < nd; i += kGT) {
             if (lay.vectors > 1) A.r[d0 + i] = vr[i];
@@ -561,7 +586,7 @@ __global__ void __launch_bounds__(kGT, 1) k_group_cg(GroupArgs<V, X> A) {
             A.S.rr[job] = rr;
             A.S.iters[job] = iters;
             A.S.status[job] = status;
-            A.S.done[job] = 1;
+            A.S.done[job] = !paused;
         }
         __syncthreads();  // shared memory is reused by the next turn
     }
@@ -987,8 +1012,14 @@ int run(nb2_ctx* c, SellPlan* P, GroupScalars S, const std::vector<int>& active,
     A.dc = dc;
     A.S = S;
     A.slots = P->slots;
+    A.failed = &c->cgs->group_failed;
+    A.launch = ++c->group_launches;
     // no value of an earlier launch carries a tag of this one
-    A.tag0 = ((unsigned long long)++P->launches << 32) + 2;
+    A.tag0 = ((unsigned long long)A.launch << 32) + 2;
+    int turns = 1;  // of one CTA
+    for (int i = 0; i < ncta; ++i)
+        turns = std::max(turns, P->h_turn_ptr[i + 1] - P->h_turn_ptr[i]);
+    A.start_limit = (int)std::min((long long)kStartLimit * turns, 1ll << 30);
     A.smem_bytes = dynamic;
     void* args[] = {&A};
     NB2_CUDA(c, cudaLaunchCooperativeKernel((const void*)kernel, dim3(ncta), dim3(kGT), args,
@@ -1031,6 +1062,8 @@ int group_cg(nb2_ctx* c, SellPlan* P, GroupScalars S, const std::vector<int>& ac
              X* p, X* q, const X* inv, const float* dc) {
     return run<V, X>(c, P, S, active, x, r, p, q, inv, dc);
 }
+bool group_failed(const nb2_ctx* c) { return c->h_cgs->group_failed == c->group_launches; }
+
 template int group_cg<double, double>(nb2_ctx*, SellPlan*, GroupScalars, const std::vector<int>&,
                                       double*, double*, double*, double*, const double*,
                                       const float*);

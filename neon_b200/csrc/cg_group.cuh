@@ -44,7 +44,6 @@ struct SellPlan {
     double* z = nullptr;             // the exchanged vector {value, tag}, 3 per row
     double* s = nullptr;             // K p of parts whose vectors do not fit in shared memory
     double* slots = nullptr;
-    unsigned launches = 0;           // part of every tag
     GroupTurn* turns = nullptr;      // device copy of the schedule
     int* turn_ptr = nullptr;
     std::vector<GroupTurn> h_turns, sent_turns;  // the schedule, and the one on the device
@@ -61,12 +60,15 @@ void sell_release(SellPlan* p);
 int sell_plan(nb2_ctx* c, const std::vector<int>& offsets, int value_bytes, SellPlan** out);
 
 // Copy the values in, rows of masked unknowns as zeros; then iterate every active job whose `done`
-// is 0 until it stops by itself (all of them when `active` is empty).  Nothing is waited for: a
-// job that is still not done once the stream is idle had a wait run out.
+// is 0 until it stops by itself or has made its iterations of one launch (all of them when `active`
+// is empty).  Nothing is waited for.  Once the stream is idle and the CG scalars are on the host
+// (wait_scalars): a job that is not done takes another launch, unless group_failed says that a wait
+// of the launch ran out, which leaves x undefined.
 template <typename V>
 int sell_fill(nb2_ctx* c, SellPlan* P, const V* K, const unsigned char* mask);
 template <typename V, typename X>
 int group_cg(nb2_ctx* c, SellPlan* P, GroupScalars S, const std::vector<int>& active, X* x, X* r,
              X* p, X* q, const X* inv, const float* dc);
+bool group_failed(const nb2_ctx* c);
 
 }  // namespace nb2

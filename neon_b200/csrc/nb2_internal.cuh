@@ -100,6 +100,7 @@ struct CgScalars {
     double rr_cap;  // mixed reliable updates: recurrence r.r above which a cycle has diverged
     int iterations, max_iterations, done, status;
     unsigned int counter[4];  // last-block tickets of the reductions
+    unsigned int group_failed;  // the last launch of the persistent PCG in which a wait ran out
 };
 
 struct Timer {
@@ -198,6 +199,7 @@ struct nb2_ctx {
     std::vector<int> sell_offsets;  // the systems it was built for (also when it came out null)
     int sms = 0;                    // 0 not asked yet, -1 no cooperative launch
     int smem_optin = 0;
+    unsigned group_launches = 0;    // its launches, part of every tag that its CTAs exchange
 
     long long launches = 0;
     std::string error;

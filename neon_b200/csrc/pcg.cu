@@ -566,8 +566,11 @@ static int run_bsr_cg(nb2_ctx* c, const V* vals, X* x, X* r, X* p, X* q, X* inv,
         CgScalars* s = c->cgs;
         const GroupScalars S{&s->threshold,  &s->abs_new, &s->beta,   &s->rr,           &s->rr_cap,
                              &s->iterations, &s->done,    &s->status, &s->max_iterations};
-        NB2_TRY((group_cg<V, X>(c, plan, S, {}, x, r, p, q, inv, nullptr)));
-        NB2_TRY(wait_scalars(c));
+        do {
+            NB2_TRY((group_cg<V, X>(c, plan, S, {}, x, r, p, q, inv, nullptr)));
+            NB2_TRY(wait_scalars(c));
+            if (group_failed(c)) return NB2_E_TIMEOUT;
+        } while (!c->h_cgs->done);
     } else {
         NB2_TRY(cg.run(maxit));
     }
