@@ -188,10 +188,11 @@ __device__ __forceinline__ void xr_one(X& x, X& r, X p, X q, X inv, X alpha, dou
     acc[1] += (double)ri * (double)(inv * ri);
 }
 
+// No __restrict__ on the vectors of the kernels that start early: they are resident while the kernel
+// ahead still writes them, and the read-only path that __restrict__ opens is for data that nothing
+// writes during a kernel's life (inv, the mask), or that the kernel itself only writes (q of the product).
 template <typename X>
-__global__ void __launch_bounds__(kRedThreads) k_xr(long long n, X* __restrict__ x,
-                                                    X* __restrict__ r, const X* __restrict__ p,
-                                                    const X* __restrict__ q,
+__global__ void __launch_bounds__(kRedThreads) k_xr(long long n, X* x, X* r, const X* p, const X* q,
                                                     const X* __restrict__ inv, CgScalars* s,
                                                     double* partials) {
     pdl_next();
@@ -247,8 +248,7 @@ __global__ void __launch_bounds__(kRedThreads) k_xr(long long n, X* __restrict__
 }
 
 template <typename X>
-__global__ void __launch_bounds__(kRedThreads) k_p(long long n, X* __restrict__ p,
-                                                   const X* __restrict__ r,
+__global__ void __launch_bounds__(kRedThreads) k_p(long long n, X* p, const X* r,
                                                    const X* __restrict__ inv, const CgScalars* s) {
     pdl_next();
     pdl_wait();
@@ -348,7 +348,7 @@ __global__ void k_copy_out(long long n, const X* __restrict__ src, double* __res
 // ---------------------------------------------------------------------------------------
 // generic CSR (drop-in linear_solver on a caller matrix)
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kRedThreads) k_csr_spmv(Csr A, const double* __restrict__ p,
+__global__ void __launch_bounds__(kRedThreads) k_csr_spmv(Csr A, const double* p,
                                                           double* __restrict__ q, CgScalars* s,
                                                           double* partials) {
     pdl_next();
@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(kRedThreads) k_csr_spmv(Csr A, const double* _
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) g[u] = c[u] >= 0 ? p[c[u]] : 0.0;
+        const double pi = lane == 0 ? p[i] : 0.0;  // in flight with the others
         double acc = 0;
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -393,7 +394,7 @@ __global__ void __launch_bounds__(kRedThreads) k_csr_spmv(Csr A, const double* _
         acc = warp_sum(acc);
         if (lane == 0) {
             q[i] = acc;
-            dot[0] += p[i] * acc;
+            dot[0] += pi * acc;
         }
         b0 = n0;
         b1 = n1;
