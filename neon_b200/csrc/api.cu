@@ -123,15 +123,24 @@ cudaError_t nb2::call_alloc(nb2_ctx* c, void** p, size_t bytes) {
         }
     }
     bytes = std::max<size_t>(bytes, 1);
-    return c->pool ? cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream) : cudaMalloc(p, bytes);
+    if (c->pool) {
+        if (cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream) == cudaSuccess) return cudaSuccess;
+        cudaGetLastError();  // the pool grows by tens of MB at a time: the bytes alone may still fit
+    }
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) c->call_plain.push_back(*p);
+    return e;
 }
 
 void nb2::call_free(nb2_ctx* c, void* p) {
     if (!p) return;
-    if (c->pool)
+    auto plain = std::find(c->call_plain.begin(), c->call_plain.end(), p);
+    if (plain == c->call_plain.end()) {
         cudaFreeAsync(p, c->stream);
-    else
-        cudaFree(p);
+        return;
+    }
+    c->call_plain.erase(plain);
+    cudaFree(p);
 }
 
 template <typename T>

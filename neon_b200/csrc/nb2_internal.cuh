@@ -117,6 +117,7 @@ struct nb2_ctx {
     bool own_stream = false;
     cudaMemPool_t pool = nullptr;  // memory of one call (call_alloc)
     bool pool_tried = false;
+    std::vector<void*> call_plain;  // ... that the pool could not give
     int device = 0;
     int N = 0, E = 0, npe = 0, nq = 0, nqp = 0, n = 0;
     long long nnzb = 0, nnz = 0;
@@ -217,7 +218,7 @@ int cuda_fail(nb2_ctx* c, cudaError_t e, const char* what);
 // Device memory that lives no longer than one call on the context, ordered on its stream.  It comes
 // from a pool of the context that keeps up to kPoolKeep bytes between calls and goes with it:
 // cudaMalloc and cudaFree wait for the device, which took 0.2 of the 5 ms of a 27-element Newton
-// solve, and now and then 0.1 to 0.9 s of a batched one.
+// solve, and now and then 0.1 to 0.9 s of a batched one.  They still serve where the pool cannot grow.
 constexpr unsigned long long kPoolKeep = 64ull << 20;
 cudaError_t call_alloc(nb2_ctx* c, void** p, size_t bytes);
 void call_free(nb2_ctx* c, void* p);
