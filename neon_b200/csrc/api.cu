@@ -924,7 +924,7 @@ struct Newton {
             c->launches++;
         }
         double* tmp = c->cg_q;  // free until the solve
-        if (mf64 || (mixed() && mf64_applies(c))) {
+        if (mf64 || (mixed() && mf64_ready(c))) {
             NB2_TRY(mf_setup(c, false, true));
             NB2_TRY(mf_apply64(c, c->inc, tmp));
         } else if (mixed())
@@ -1082,7 +1082,8 @@ extern "C" int nb2_static_solve(nb2_ctx* c, const nb2_solver_options* options,
     }
     if (nw.o.precision == NB2_MIXED) {
         NB2_TRY(ensure_cg32(c));
-        NB2_TRY(ensure_mf(c, true, true));
+        NB2_TRY(ensure_mf(c, true, false));
+        ensure_mf(c, false, true);  // the FP64 residual's operator, optional
         if (!(nw.o.mixed_inner_tolerance > 0)) nw.o.mixed_inner_tolerance = 1e-4;
     } else {
         NB2_TRY(ensure_k64(c));

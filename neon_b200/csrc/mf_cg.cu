@@ -24,6 +24,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <exception>
+#include <string>
+
 #include <thrust/device_ptr.h>
 #include <thrust/execution_policy.h>
 #include <thrust/sort.h>
@@ -901,16 +904,20 @@ int build_plan(nb2_ctx* c, MfPlan* P) {
     NB2_TRY(allocate(c, &P->de, 3 * m));
     // node -> its products, ascending (a stable sort keeps it)
     Scratch keys;
-    NB2_CUDA(c, cudaMalloc(&keys.p, sizeof(int) * m));
-    auto* kp = static_cast<int*>(keys.p);
-    if (npe == 8)
-        k_product_nodes<8><<<element_grid(c), element_threads(c), 0, c->stream>>>(E, N, c->conn, kp, P->nidx);
-    else
-        k_product_nodes<4><<<element_grid(c), element_threads(c), 0, c->stream>>>(E, N, c->conn, kp, P->nidx);
-    auto pol = thrust::cuda::par.on(c->stream);
-    thrust::stable_sort_by_key(pol, thrust::device_pointer_cast(kp),
-                               thrust::device_pointer_cast(kp + m),
-                               thrust::device_pointer_cast(P->nidx));
+    int* kp = nullptr;
+    NB2_TRY(allocate(c, &kp, m));
+    keys.p = kp;
+    auto product_nodes = npe == 8 ? k_product_nodes<8> : k_product_nodes<4>;
+    product_nodes<<<element_grid(c), element_threads(c), 0, c->stream>>>(E, N, c->conn, kp, P->nidx);
+    try {  // its scratch may not fit; no exception may pass the C interface
+        thrust::stable_sort_by_key(thrust::cuda::par.on(c->stream), thrust::device_pointer_cast(kp),
+                                   thrust::device_pointer_cast(kp + m),
+                                   thrust::device_pointer_cast(P->nidx));
+    } catch (const std::exception& e) {
+        cudaGetLastError();
+        c->error = std::string("matrix-free operator: ") + e.what();
+        return NB2_E_CUDA;
+    }
     k_node_products<<<(N + 1 + 255) / 256, 256, 0, c->stream>>>(kp, P->nidx, m, N, P->first,
                                                                P->nptr);
     c->launches += 2;
@@ -1034,6 +1041,10 @@ void mf_release(MfPlan* P) {
 
 bool mf64_applies(const nb2_ctx* c) { return !model_aniso(c->mat.model); }
 
+bool mf64_ready(const nb2_ctx* c) {
+    return c->mf && c->mf->mc64 && c->mf->x && c->mf->z64;
+}
+
 int ensure_mf(nb2_ctx* c, bool fp32, bool fp64) {
     if (!c->mf) {
         auto* P = new MfPlan();
@@ -1052,10 +1063,21 @@ int ensure_mf(nb2_ctx* c, bool fp32, bool fp64) {
         NB2_TRY(allocate(c, &P->z32, 4ll * c->N));
         NB2_TRY(allocate(c, &P->p32, 4ll * c->N));
     }
-    if (fp64 && mf64_applies(c)) {
-        NB2_TRY(allocate(c, &P->mc64, points));
-        NB2_TRY(allocate(c, &P->x, (long long)c->n));
-        NB2_TRY(allocate(c, &P->z64, (long long)c->n));
+    if (fp64 && mf64_applies(c) && !mf64_ready(c)) {
+        int st = allocate(c, &P->mc64, points);
+        if (st == NB2_OK) st = allocate(c, &P->x, (long long)c->n);
+        if (st == NB2_OK) st = allocate(c, &P->z64, (long long)c->n);
+        if (st != NB2_OK) {  // its callers go without it: leave them the room
+            for (double** p : {&P->mc64, &P->x, &P->z64}) {
+                if (*p) cudaFree(*p);
+                *p = nullptr;
+            }
+            if (!P->p32) {
+                mf_release(P);
+                c->mf = nullptr;
+            }
+            return st;
+        }
     }
     return NB2_OK;
 }
@@ -1127,8 +1149,8 @@ int pcg_mf64(nb2_ctx* c, const double* b, double* x, double tol, int maxit, int*
 // linear_solver.cpp:67-109).
 int pcg_reliable_mixed(nb2_ctx* c, const double* b, double* x, double tol, double delta,
                        int maxit, double* work, int* iterations, bool use_graphs) {
-    const bool mf64 = mf64_applies(c);
-    NB2_TRY(ensure_mf(c, true, mf64));
+    const bool mf64 = mf64_ready(c);  // else the element kernels' product
+    NB2_TRY(ensure_mf(c, true, false));
     MfPlan* P = c->mf;
     NB2_TRY(mf_setup(c, true, mf64));
     NB2_TRY(jacobi(c, c->cg32_inv));

@@ -23,8 +23,10 @@ struct MfPlan {
 
 void mf_release(MfPlan* p);
 
-// Build the plan (once per context) and the buffers of the FP32 and / or FP64 operator.
+// Build the plan (once per context) and the buffers of the FP32 and / or FP64 operator.  Where the
+// memory does not suffice nothing of the FP64 operator is left allocated: solves go without it.
 int ensure_mf(nb2_ctx* c, bool fp32, bool fp64);
+bool mf64_ready(const nb2_ctx* c);  // the FP64 operator's buffers are there
 // whether the FP64 operator exists for the context's model (the anisotropic microspheres keep
 // the assembled K: 29 FP64 coefficients per point are as many bytes)
 bool mf64_applies(const nb2_ctx* c);
@@ -40,7 +42,7 @@ int mf_apply(nb2_ctx* c, const double* v, double* y);
 int pcg_mf64(nb2_ctx* c, const double* b, double* x, double tol, int maxit, int* iterations,
              double* error, bool use_graphs);
 // mixed precision with reliable updates: FP32 iterations, FP64 true residual every `delta`
-// reduction; work: n doubles
+// reduction (on the FP64 operator where it is ready); work: n doubles
 int pcg_reliable_mixed(nb2_ctx* c, const double* b, double* x, double tol, double delta,
                        int maxit, double* work, int* iterations, bool use_graphs);
 

@@ -1,6 +1,6 @@
-"""Newton solves that run out of device memory for what they can do without: growth of the pool that a
-call's memory comes from, the tiled copy of K.  They take the path that needs less and reach the same
-solution, to the 1e-8 between two paths of the other tests.
+"""Newton solves that run out of device memory for what they can do without: the matrix-free operator (its
+plan, the scratch of its sort, its coefficients), the tiled copy of K, the second K buffer.  They take
+the path that needs less and reach the same solution, to the 1e-8 between two paths of the other tests.
 
 A child process fills the device but for a given number of MB before each solve; its kernels are loaded
 up front, since loading one needs memory too."""
@@ -62,3 +62,8 @@ def test_small_solve_beside_a_full_device():
     """A few hundred KB are enough for what a call of this size allocates."""
     _run("fp64", (6, 7, 5), (6, 12, 24))
 
+
+@pytest.mark.parametrize("precision,left", [("fp64", (16, 24, 26, 28, 30, 40, 56, 72)),
+                                            ("mixed", (64, 72, 80, 88, 96))])
+def test_matrix_free_solve_with_little_memory(precision, left):
+    _run(precision, (41, 37, 39), left)
