@@ -1301,7 +1301,8 @@ static void mf_setup_t(nb2_ctx* c, const ElementArgs& A, float* md,
                        R* mc, double* de) {
     constexpr int EPC = Topo<NPE>::EPC, G = Topo<NPE>::G;
     const unsigned grid = (unsigned)((c->E + EPC - 1) / EPC);
-    k_mf_setup<NPE, MODEL, R><<<grid, EPC * G, 0, c->stream>>>(A, md, mc, de);
+    k_mf_setup<NPE, MODEL, R><<<grid, EPC * G, 0, c->stream>>>(A, md, mc, de, &c->cgs->mf_odd_setup,
+                                                               c->mf_setups);
     c->launches++;
 }
 
@@ -1333,6 +1334,7 @@ int launch_mf_setup32(nb2_ctx* c, float* md, float* mc,
                       double* de) {
     NB2_TRY(upload_tables(c));
     if (!c->dpar || !c->u_tan) return NB2_E_INPUT;
+    ++c->mf_setups;
     return c->npe == 8 ? mf_setup_model<8>(c, md, mc, de)
                        : mf_setup_model<4>(c, md, mc, de);
 }

@@ -855,7 +855,10 @@ cudaError_t apply_model(nb2_ctx* c, bool pdl, const R* z, const R* p, const CgSc
     switch (c->mat.model) {
         case MODEL_LE: return apply_t<NPE, MODEL_LE>(c, pdl, z, p, s);
         case MODEL_NH: return apply_t<NPE, MODEL_NH>(c, pdl, z, p, s);
-        case MODEL_J2: return apply_t<NPE, MODEL_J2>(c, pdl, z, p, s);
+        case MODEL_J2:
+            if constexpr (sizeof(R) == 4)
+                if (!c->mf->odd32) return apply_t<NPE, MODEL_J2>(c, pdl, z, p, s);
+            return apply_t<NPE, MODEL_J2S>(c, pdl, z, p, s);
         case MODEL_MS: return apply_t<NPE, MODEL_MS>(c, pdl, z, p, s);
         default:
             if constexpr (sizeof(R) == 4)
@@ -1029,8 +1032,8 @@ struct MfRunner {
 
 void mf_release(MfPlan* P) {
     if (!P) return;
-    if (P->graph32) cudaGraphExecDestroy(P->graph32);
-    if (P->graph64) cudaGraphExecDestroy(P->graph64);
+    for (auto g : {P->graph32[0], P->graph32[1], P->graph64})
+        if (g) cudaGraphExecDestroy(g);
     void* ptrs[] = {P->first, P->nptr, P->nidx, P->ye,  P->de, P->md,
                     P->mc32,  P->mc64, P->x,    P->z32, P->p32,
                     P->z64};
@@ -1094,6 +1097,13 @@ int mf_setup(nb2_ctx* c, bool fp32, bool fp64) {
     return NB2_OK;
 }
 
+// which FP32 product the last setup asks for; waits for it
+static int choose_product32(nb2_ctx* c) {
+    NB2_TRY(wait_scalars(c));
+    c->mf->odd32 = c->h_cgs->mf_odd_setup == c->mf_setups;
+    return NB2_OK;
+}
+
 int mf_apply64(nb2_ctx* c, const double* v, double* y) {
     const double* none = nullptr;
     NB2_CUDA(c, apply<double>(c, false, v, none, nullptr));
@@ -1107,6 +1117,7 @@ int mf_apply64(nb2_ctx* c, const double* v, double* y) {
 int mf_apply(nb2_ctx* c, const double* v, double* y) {
     NB2_TRY(ensure_mf(c, true, false));
     NB2_TRY(mf_setup(c, true, false));
+    NB2_TRY(choose_product32(c));
     k_to_float<<<vec_grid(c->n), 256, 0, c->stream>>>(c->n, v, c->mf->z32);
     const float* none = nullptr;
     NB2_CUDA(c, apply<float>(c, false, (const float*)c->mf->z32, none, nullptr));
@@ -1155,7 +1166,7 @@ int pcg_reliable_mixed(nb2_ctx* c, const double* b, double* x, double tol, doubl
     NB2_TRY(mf_setup(c, true, mf64));
     NB2_TRY(jacobi(c, c->cg32_inv));
     MfRunner<float> cg{c,         c->cg32_x,   c->cg32_r,  P->z32,     P->p32,
-                       c->cg32_q, c->cg32_inv, use_graphs, &P->graph32};
+                       c->cg32_q, c->cg32_inv, use_graphs, nullptr};
     const long long n = c->n;
     const int RB = reduction_blocks(c);
     NB2_CUDA(c, cudaMemsetAsync(x, 0, sizeof(double) * n, c->stream));
@@ -1164,7 +1175,8 @@ int pcg_reliable_mixed(nb2_ctx* c, const double* b, double* x, double tol, doubl
                                                         c->cgs, c->partials, std::max(tol, delta),
                                                         maxit);
     c->launches++;
-    NB2_TRY(wait_scalars(c));
+    NB2_TRY(choose_product32(c));
+    cg.cache = &P->graph32[P->odd32];
     const double b2 = c->h_cgs->rhs_norm2;
     const double thr = std::max(tol * tol * b2, 2.2250738585072014e-308);
     *iterations = 0;

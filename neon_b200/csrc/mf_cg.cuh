@@ -18,7 +18,8 @@ struct MfPlan {
     double* x = nullptr;
     float *z32 = nullptr, *p32 = nullptr;  // D^-1 r and p of the PCG ([N][4]; FP64: [N][3])
     double* z64 = nullptr;
-    cudaGraphExec_t graph32 = nullptr, graph64 = nullptr;
+    cudaGraphExec_t graph32[2] = {nullptr, nullptr}, graph64 = nullptr;  // FP32: by odd32
+    bool odd32 = false;                    // the last FP32 setup needs MODEL_J2S
 };
 
 void mf_release(MfPlan* p);

@@ -17,12 +17,13 @@
 //                    s = w det J comes from the element's own geometry at apply time.  Six numbers
 //                    per point instead of nine, one at an elastic point.  A softening material
 //                    leaves that range (b > 0 where the yield stress of the last state is
-//                    negative, mu' < 0 where the present one is): such a point stores -infinity,
-//                    N, mu' and b.
+//                    negative, mu' < 0 where the present one is): such a point stores
+//                    -kOddPoint, N, mu' and b, and leaves this setup's number in *odd_setup.
 //   de[3a+i][e]      = element contribution to K_(3a+i, 3a+i)
 template <int NPE, int MODEL, typename R>
 __global__ void __launch_bounds__(64) k_mf_setup(ElementArgs A, float* __restrict__ md,
-                                                 R* __restrict__ mc, double* __restrict__ de) {
+                                                 R* __restrict__ mc, double* __restrict__ de,
+                                                 unsigned* odd_setup, unsigned setup) {
     using T = Topo<NPE>;
     constexpr int NQ = T::NQ, G = T::G, EPC = T::EPC;
     constexpr bool kFinite = (MODEL == MODEL_NH || MODEL == MODEL_MS || model_aniso(MODEL));
@@ -84,10 +85,10 @@ __global__ void __launch_bounds__(64) k_mf_setup(ElementArgs A, float* __restric
             for (int c = 0; c < 6; ++c) N6[c] = A.dpar[(3 + c) * n + q];
             const R mu_r = (R)mu;
             const bool plastic = b != 0.0;
-            // what the short form cannot hold: a sign of its own, an infinity, NaN
-            const bool odd = plastic ? !(b < 0.0 && mu_r > (R)0 && mu_r < (R)INFINITY) : mu_r < (R)0;
+            // what the short form cannot hold: signs of their own, NaN at a plastic point
+            const bool odd = plastic ? !(b < 0.0 && mu_r > kOddPoint<R>) : mu_r < (R)0;
             const double f = odd ? 1.0 : (plastic ? sqrt(-b) : 0.0);
-            near[0] = odd ? -(R)INFINITY : (plastic ? -mu_r : mu_r);
+            near[0] = odd ? -kOddPoint<R> : (plastic ? -mu_r : mu_r);
             far[0 * n] = (R)(f * N6[0]);
             far[1 * n] = (R)(f * N6[1]);
             far[2 * n] = (R)(f * N6[3]);
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(64) k_mf_setup(ElementArgs A, float* __restric
             if (odd) {
                 far[5 * n] = mu_r;
                 far[6 * n] = (R)b;
+                *(volatile unsigned*)odd_setup = setup;
             }
         } else {
             near[0] = (R)(s * lam);

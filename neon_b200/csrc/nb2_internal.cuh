@@ -101,6 +101,7 @@ struct CgScalars {
     int iterations, max_iterations, done, status;
     unsigned int counter[4];  // last-block tickets of the reductions
     unsigned int group_failed;  // the last launch of the persistent PCG in which a wait ran out
+    unsigned int mf_odd_setup;  // the last FP32 setup of the matrix-free operator with a MODEL_J2S point
 };
 
 struct Timer {
@@ -201,6 +202,7 @@ struct nb2_ctx {
     int sms = 0;                    // 0 not asked yet, -1 no cooperative launch
     int smem_optin = 0;
     unsigned group_launches = 0;    // its launches, part of every tag that its CTAs exchange
+    unsigned mf_setups = 0;         // FP32 setups of the matrix-free operator
 
     long long launches = 0;
     std::string error;

@@ -607,9 +607,10 @@ void release_graphs(nb2_ctx* c) {
     if (c->graph32) cudaGraphExecDestroy(c->graph32);
     c->graph32 = nullptr;
     if (c->mf) {
-        if (c->mf->graph32) cudaGraphExecDestroy(c->mf->graph32);
-        if (c->mf->graph64) cudaGraphExecDestroy(c->mf->graph64);
-        c->mf->graph32 = c->mf->graph64 = nullptr;
+        for (auto* g : {&c->mf->graph32[0], &c->mf->graph32[1], &c->mf->graph64}) {
+            if (*g) cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
     }
 }
 

@@ -3,11 +3,12 @@ modulus mu' = G sigma_y / q is negative where the yield stress of the present st
 where that of the last one is; the operators have to be the assembled K there too.
 
 FP32: the product against the assembled K, to the rounding bar of the FP32 product's other tests.
-FP64: a Newton solve past the size that runs matrix-free, with every DOF prescribed but those of a few
-interior nodes (a linear system that CG solves exactly whatever its signs), against the same Newton
-steps with the downloaded K and a dense solve.  Both solve the same linear systems, CG to 1e-12, so the
-norms of the log agree to 1e-8 relative while they are within 1e-6 of the largest (1e-12 of rounding
-over 1e-6, with a factor of 100 for the Newton map), and the displacements to 1e-10."""
+Newton solves, FP64 and mixed (whose residuals are FP64): past the size that runs matrix-free, with every
+DOF prescribed but those of a few interior nodes (a linear system that CG solves exactly whatever its
+signs), against the same Newton steps with the downloaded K and a dense solve.  Both solve the same linear
+systems, CG to 1e-12, so the norms of the log agree to 1e-8 relative while they are within 1e-6 of the
+largest (1e-12 of rounding over 1e-6, with a factor of 100 for the Newton map), and the displacements to
+1e-10."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -111,11 +112,12 @@ def _reference(api, pr, free):
     return u, np.array(log)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("hardening", [1e3, -1e5])
-def test_fp64_newton_at_plastic_points(api, hardening):
+def test_newton_at_plastic_points(api, hardening, precision):
     pr, free = _prescribed(hardening)
     ur, ref = _reference(api, pr, free)
-    sm = api.StaticMatrix(pr)
+    sm = api.StaticMatrix(pr, precision=api.MIXED if precision == "mixed" else api.FP64)
     u = sm.solve(raise_on_error=False)
     got = sm.log[:len(ref), 3:5]
     far = ref > 1e-6 * ref.max(0)
