@@ -864,7 +864,7 @@ struct Newton {
         if (!k_pending) return NB2_OK;
         k_pending = false;
         std::swap(c->u, c->u_tan);
-        const int st = launch_element_kernel(c, MODE_STIFFNESS | MODE_FORCE, NB2_FP64);
+        const int st = launch_element_kernel(c, MODE_STIFFNESS | MODE_FORCE, NB2_FP64, true);
         std::swap(c->u, c->u_tan);
         return st;
     }

@@ -1445,7 +1445,7 @@ static bool colour_applies(const nb2_ctx* c, int mode, int precision) {
     return true;
 }
 
-int launch_element_kernel(nb2_ctx* c, int mode, int precision) {
+int launch_element_kernel(nb2_ctx* c, int mode, int precision, bool one_buffer) {
     int st = upload_tables(c);
     if (st) return st;
     bool coloured = false;
@@ -1455,8 +1455,10 @@ int launch_element_kernel(nb2_ctx* c, int mode, int precision) {
     }
     // FP64 K of one problem is double-buffered: the buffer zeroed in the background during the
     // previous pass becomes K, and the previous K is zeroed during this pass (it is no longer
-    // read once the work queued before this pass is done)
-    const bool kdouble = (mode & MODE_STIFFNESS) && precision == NB2_FP64 && !c->e_inst;
+    // read once the work queued before this pass is done).  Not for an assembly that stands alone
+    // (one_buffer): the next one is far off.
+    const bool kdouble =
+        (mode & MODE_STIFFNESS) && precision == NB2_FP64 && !c->e_inst && !one_buffer;
     if (kdouble) NB2_TRY(ensure_k64_alt(c));
     const bool kbg = kdouble && c->kalt_state == 1;
     if (mode & MODE_STIFFNESS) {

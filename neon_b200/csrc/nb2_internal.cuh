@@ -252,7 +252,7 @@ int ensure_colouring(nb2_ctx* c);      // element colours and the colour-sorted 
 int export_csr_values(nb2_ctx* c, const double* Kbsr, double* Kcsr_dev);
 
 // elements.cu
-int launch_element_kernel(nb2_ctx* c, int mode, int precision);
+int launch_element_kernel(nb2_ctx* c, int mode, int precision, bool one_buffer = false);
 int launch_apply(nb2_ctx* c, const double* v, double* y);  // y = K v, FP64 matrix-free
 int launch_element_stiffness(nb2_ctx* c, long long e, double* Ke_dev);  // one dense K_e
 int launch_adjoint_shear(nb2_ctx* c, const double* lam, double* dJdG);

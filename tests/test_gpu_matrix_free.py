@@ -90,3 +90,22 @@ def test_the_resident_stiffness_after_a_matrix_free_solve(api):
     K0, _ = g.assemble()
     assert rel_err(K, K0) < 1e-8  # K moves with u, which the last Newton step changes by 1e-8
     assert np.array_equal(u, sm.mesh.displacement())
+
+
+def test_a_matrix_free_solve_needs_no_second_k_buffer(api):
+    """The FP64 K buffer that is zeroed in the background is for assemblies that follow one another; the
+    one assembly at the end of an increment goes without.  Free memory falls by that buffer with the
+    first assembling pass afterwards, not with the solve."""
+    import torch
+    pr = _problem("neohooke", M.structured_hex8(41, 37, 39))
+    sm = api.StaticMatrix(pr)
+    sm.solve()
+    after_solve = torch.cuda.mem_get_info()[0]
+    sm.mesh.update_assemble_device()
+    sm.mesh.synchronize()
+    k_bytes = 72 * sm.mesh.nnzb
+    assert after_solve - torch.cuda.mem_get_info()[0] >= 0.9 * k_bytes
+    K, _ = sm.mesh.download_system(K=True, f=False)
+    sm.mesh.update_assemble_device()  # the other buffer
+    K1, _ = sm.mesh.download_system(K=True, f=False)
+    assert rel_err(K1, K) < 1e-13  # the order of atomic additions
