@@ -41,7 +41,7 @@ namespace {
 
 // threads of an element block: a hex8 thread runs long, so small blocks fill the last wave better
 template <int NPE>
-constexpr int kThreads = NPE == 8 ? 64 : 256;
+constexpr int kThreads = NPE == 8 ? 64 : 128;
 constexpr int kIterations = 32;  // CG iterations per captured graph
 
 // ---------------------------------------------------------------------------------------
@@ -357,12 +357,14 @@ __device__ __forceinline__ void element_product(const R (&d)[NPE][3], const R (&
     }
 }
 
-// CTAs per SM that the registers are cut for (64 threads each).  FP32: 8 (128 registers); J2, which
+// CTAs per SM that the registers are cut for (hex8: 64 threads each).  FP32: 8 (128 registers); J2, which
 // needs the fewest, 10 (96, a few spilled): 141 against 145 us per iteration at 100^3, and 163 with 6;
-// finite strain at 64^3 56 us with 8, 59 with 6, 61 with 10.
+// finite strain at 64^3 56 us with 8, 59 with 6, 61 with 10.  tet4 (128 threads each) waits for memory, so
+// warps count: 10 (48 registers), 8 for the anisotropic models.  72^3 x 6 linear, neo-Hooke, Langevin: 113,
+// 114, 140 us per iteration; 116, 117, 144 with 4 of 256 threads (56 to 72 registers).
 template <int NPE, int MODEL, typename R>
 constexpr int apply_blocks() {
-    if (NPE == 4) return sizeof(R) == 8 || model_aniso(MODEL) ? 2 : 4;
+    if (NPE == 4) return sizeof(R) == 8 ? 4 : (model_aniso(MODEL) ? 8 : 10);
     return sizeof(R) == 8 || model_aniso(MODEL) ? 4 : (MODEL == MODEL_J2 ? 10 : 8);
 }
 
@@ -411,8 +413,12 @@ __global__ void __launch_bounds__(kThreads<NPE>, apply_blocks<NPE, MODEL, R>())
     R v[NPE][3], y[NPE][3], beta = (R)0;
     int done = 0;
     if (s) {
-        done = *reinterpret_cast<const volatile int*>(&s->done);
-        beta = (R) * reinterpret_cast<const volatile double*>(&s->beta);
+        // through L1 (a volatile load is not): every warp reads this one line, and 50,000 of them
+        // at one L2 slice took 9 of 42 us for tet4 at 64^3
+        double b;
+        asm volatile("ld.global.s32 %0, [%1];" : "=r"(done) : "l"(&s->done) : "memory");
+        asm volatile("ld.global.f64 %0, [%1];" : "=d"(b) : "l"(&s->beta) : "memory");
+        beta = (R)b;
     }
 #pragma unroll
     for (int a = 0; a < NPE; ++a) load_node_now(z, nd[a], v[a]);
