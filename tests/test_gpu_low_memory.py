@@ -48,22 +48,67 @@ print("complete")
 """
 
 
-def _run(precision, shape, left):
+BATCH = """
+import sys
+import ctypes as C
+import numpy as np
+import torch
+from conftest import rel_err
+from neon_b200 import api, problem as P
+
+problems = [P.config_c5_instance(m, mu, increments=1) for m, mu in ((24, 0.7), (23, 1.9), (22, 1.2))]
+for pr in problems:
+    pr.options.residual_tolerance = pr.options.displacement_tolerance = 1e-8
+precision = api.MIXED if sys.argv[1] == "mixed" else api.FP64
+ref = api.BatchedStaticMatrix(problems, precision=precision, autotune=False)
+
+def launches(g):
+    n = C.c_int64()
+    api.lib().nb2_launch_count(g.h, C.byref(n))
+    return n.value
+
+u0 = ref.solve()
+few = launches(ref.mesh)
+ref.mesh.close()
+b = api.BatchedStaticMatrix(problems, precision=precision, autotune=False)
+b.mesh.update_assemble_device(precision)
+b.mesh.synchronize()
+free = torch.cuda.mem_get_info()[0]
+fill = torch.empty(free - (int(sys.argv[2]) << 20), dtype=torch.uint8, device="cuda")
+u = b.solve()
+many = launches(b.mesh)
+for i in range(3):
+    e = rel_err(b.instance_displacement(i, u), ref.instance_displacement(i, u0))
+    print(i, e, b.reports[i]["cg_iterations"], ref.reports[i]["cg_iterations"], few, many, flush=True)
+    assert e < 1e-8
+    assert abs(b.reports[i]["cg_iterations"] / ref.reports[i]["cg_iterations"] - 1) < 0.05
+assert many > 3 * few
+print("complete")
+"""
+
+
+def _run(code, precision, *args):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     env = dict(os.environ, CUDA_MODULE_LOADING="EAGER",
                PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
-    r = subprocess.run([sys.executable, "-c", CHILD, precision, ",".join(map(str, shape)),
-                        *map(str, left)], cwd=root, env=env, capture_output=True, text=True,
+    r = subprocess.run([sys.executable, "-c", code, precision, *args], cwd=root, env=env, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "complete" in r.stdout, r.stdout + r.stderr
 
 
 def test_small_solve_beside_a_full_device():
     """A few hundred KB are enough for what a call of this size allocates."""
-    _run("fp64", (6, 7, 5), (6, 12, 24))
+    _run(CHILD, "fp64", "6,7,5", "6", "12", "24")
 
 
 @pytest.mark.parametrize("precision,left", [("fp64", (16, 24, 26, 28, 30, 40, 56, 72)),
                                             ("mixed", (64, 72, 80, 88, 96))])
 def test_matrix_free_solve_with_little_memory(precision, left):
-    _run(precision, (41, 37, 39), left)
+    _run(CHILD, precision, "41,37,39", *map(str, left))
+
+
+@pytest.mark.parametrize("precision,left", [("fp64", 44), ("mixed", 36)])
+def test_batch_without_the_tiled_copy(precision, left):
+    """The copy of K that the persistent PCG reads (about 60 MB here, 35 in FP32) does not fit: the chunk
+    kernels solve the batch, with the same iterations but for the order of sums."""
+    _run(BATCH, precision, str(left))
