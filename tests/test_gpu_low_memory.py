@@ -71,6 +71,7 @@ u0 = ref.solve()
 few = launches(ref.mesh)
 ref.mesh.close()
 b = api.BatchedStaticMatrix(problems, precision=precision, autotune=False)
+b.mesh.update_internal_variables(np.zeros(b.mesh.ndofs))
 b.mesh.update_assemble_device(precision)
 b.mesh.synchronize()
 free = torch.cuda.mem_get_info()[0]
@@ -91,24 +92,24 @@ def _run(code, precision, *args):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     env = dict(os.environ, CUDA_MODULE_LOADING="EAGER",
                PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
-    r = subprocess.run([sys.executable, "-c", code, precision, *args], cwd=root, env=env, capture_output=True, text=True,
-                       timeout=300)
+    r = subprocess.run([sys.executable, "-c", code, precision, *args], cwd=root, env=env,
+                       capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "complete" in r.stdout, r.stdout + r.stderr
 
 
 def test_small_solve_beside_a_full_device():
     """A few hundred KB are enough for what a call of this size allocates."""
-    _run(CHILD, "fp64", "6,7,5", "6", "12", "24")
+    _run(CHILD, "fp64", "6,7,5", "12", "20", "28")
 
 
-@pytest.mark.parametrize("precision,left", [("fp64", (16, 24, 26, 28, 30, 40, 56, 72)),
+@pytest.mark.parametrize("precision,left", [("fp64", (20, 24, 26, 28, 30, 40, 56, 72)),
                                             ("mixed", (64, 72, 80, 88, 96))])
 def test_matrix_free_solve_with_little_memory(precision, left):
     _run(CHILD, precision, "41,37,39", *map(str, left))
 
 
-@pytest.mark.parametrize("precision,left", [("fp64", 44), ("mixed", 36)])
+@pytest.mark.parametrize("precision,left", [("fp64", 30), ("mixed", 22)])
 def test_batch_without_the_tiled_copy(precision, left):
-    """The copy of K that the persistent PCG reads (about 60 MB here, 35 in FP32) does not fit: the chunk
+    """The copy of K that the persistent PCG reads (54 MB here, 27 in FP32) does not fit: the chunk
     kernels solve the batch, with the same iterations but for the order of sums."""
     _run(BATCH, precision, str(left))
