@@ -370,9 +370,11 @@ int nb2_batch_static_solve(nb2_ctx* ctx, int32_t num_instances, const int32_t* n
                            const int32_t* dirichlet_offsets, const nb2_dof_table* nodal_forces,
                            const int32_t* force_offsets, double* u_out,
                            nb2_solve_report* reports, nb2_newton_log* log, int32_t max_log);
-/* Autotuner of the batched PCG: times the SpMV over the instances' rows for each rows-per-chunk
- * (16, 32, 64, 128) and lanes-per-block-row (4, 8, 16, 32) candidate on this device and keeps
- * the fastest for the context's next nb2_batch_static_solve.  No counterpart in the reference. */
+/* Autotuner of the batched PCG's chunk kernels: times the SpMV over the instances' rows for each
+ * rows-per-chunk (16, 32, 64, 128) and lanes-per-block-row (4, 8, 16, 32) candidate on this device and
+ * keeps the fastest for the context's next nb2_batch_static_solve.  A batch whose linear solves run in
+ * the persistent PCG (most do) uses the row chunks in its vector work only; the choice matters where
+ * that PCG's plan does not apply.  No counterpart in the reference. */
 int nb2_batch_autotune(nb2_ctx* ctx, int32_t num_instances, const int32_t* node_offsets,
                        int32_t precision, int32_t* rows_per_chunk, int32_t* lanes_per_row,
                        double* ms_per_spmv);

@@ -545,7 +545,8 @@ class BatchedStaticMatrix:
         return len(self.problems)
 
     def autotune(self):
-        """Pick the batched PCG's rows per chunk and lanes per block row by timing."""
+        """Pick rows per chunk and lanes per block row of the batched PCG's chunk kernels by timing (they
+        run where the persistent PCG's plan does not apply)."""
         R, L, ms = C.c_int32(), C.c_int32(), C.c_double()
         _check(lib().nb2_batch_autotune(self.mesh.h, self.num_instances,
                                         self.node_offsets.ctypes.data, int(self.precision),

@@ -537,8 +537,7 @@ int nb2_pcg_solve(int32_t n, const int32_t* rowptr, const int32_t* col, const do
                   double* error) {
     if (n <= 0 || !rowptr || !col || !values || !b || !x || maxit <= 0) return NB2_E_INPUT;
     // the device kernels index x[col[k]] and rows rowptr[i]..rowptr[i+1]: validated first, the columns
-    // on the device
-    // (here only if the device could not be asked)
+    // on the device (here only if the device could not be asked)
     if (rowptr[0] != 0) return NB2_E_INPUT;
     for (int i = 0; i < n; ++i)
         if (rowptr[i + 1] < rowptr[i]) return NB2_E_INPUT;
@@ -770,12 +769,13 @@ extern "C" int nb2_adjoint_shear_gradient(nb2_ctx* c, const double* dJdu, int32_
 // ---------------------------------------------------------------------------------------
 namespace {
 
-// Whether the assembled K fits in L2 (126 MB, with room for the vectors).  A Newton solve then runs
-// on it in one persistent launch per linear solve (cg_group.cu), also when mixed precision is asked
-// for: FP64 is the faster of the two there (37x29x32 neo-Hooke, 77 MB: 12 us per iteration against
-// 22 in FP32 matrix-free; 20^3: 6 against 18; tet4 48^3 x 6, 127 MB: 38 against 45).  Larger hex8
-// solves run on the matrix-free operator in either precision (FP64 at 40^3, 141 MB: 32 us against
-// 34; 48^3: 46 against 66; 64^3: 92 against 124; 100^3: 219 against 450).
+// Whether the assembled K is in L2 (126 MB) for most of an iteration.  A Newton solve then runs on it
+// in one persistent launch per linear solve (cg_group.cu), also when mixed precision is asked for.
+// The line is where FP64 stops being the faster of the two: tet4, whose rows have 15 blocks and little
+// padding, is ahead a little beyond the L2 size, hex8 not up to it (37x29x32 neo-Hooke, 77 MB: 12 us
+// per iteration against 22 in FP32 matrix-free; 20^3: 6 against 18; tet4 48^3 x 6, 127 MB: 38 against
+// 45).  Larger hex8 solves run on the matrix-free operator in either precision (FP64 at 40^3, 141 MB:
+// 30 us against 34 on the assembled K; 48^3: 42 against 66; 64^3: 90 against 124; 100^3: 216 against 450).
 static bool k_in_l2(const nb2_ctx* c) {
     return 72.0 * (double)c->nnzb <= (c->npe == 8 ? 100e6 : 130e6);
 }
@@ -1072,8 +1072,8 @@ extern "C" int nb2_static_solve(nb2_ctx* c, const nb2_solver_options* options,
     nw.o = *options;
     if (nw.o.linear_iterations <= 0 || nw.o.cg_maximum_iterations <= 0) return NB2_E_INPUT;
     // the context's solver buffers (kept for later solves) are set up before the clock of the
-    // report starts.  The mixed path assembles no K: its PCG runs on the FP32 matrix-free
-    // operator, so it needs the FP32 vectors and that operator's buffers, not K32
+    // report starts.  A mixed solve beyond the FP64 rule (k_in_l2) assembles no K: its PCG runs on the
+    // FP32 matrix-free operator, so it needs the FP32 vectors and that operator's buffers, not K32
     NB2_TRY(ensure_split_buffers(c));
     if (nw.o.precision == NB2_MIXED && k_in_l2(c)) {
         SellPlan* plan = nullptr;

@@ -24,15 +24,15 @@
 // The textbook form sums twice (p.q, then r.r and r.z); what the second sum costs is latency, the same
 // at every size: 6.0 -> 5.0 us per iteration at 12^3 hex8 cells, 6.6 -> 5.6 at 20^3, 10.6 -> 9.4 at
 // 28^3, 11.6 -> 11.7 at 37x29x32 (two more vectors in shared memory leave less room for K), with the
-// iteration counts and the errors of before.  The first iteration of
-// a launch takes the textbook form (s = K p, p.s), because its p may carry on from an earlier launch.
+// iteration counts and the errors of before (now 4.8, 5.4, 9.1 and 11.4: fewer exchanges in a sum).  The first iteration of a launch takes the textbook form
+// (s = K p, p.s), because its p may carry on from an earlier launch.
 // In the sum every member adds the same numbers in the same order: all take the same decision and a
-// solve is bit-reproducible.  Members exchange partial sums and z as 16-byte {value, tag} pairs, written and read in one access: a reader waits for the tag
-// it expects, so nothing needs a fence or a separate barrier.  A z is overwritten only after the
-// sum that follows it, to which every reader contributes after its reads.  Sums go over m1 CTAs, then over
-// m2 such groups (a push to each peer's own slots): 2.1 k cycles for up to 16 CTAs and 3.6 k for
-// 144, where an arrival count with release and acquire took 3.8 k and 4.8 k, and polling all
-// partials in one place 9.8 k (every SM then polls the same 37 lines).
+// solve is bit-reproducible.  Members exchange partial sums and z as 16-byte {value, tag} pairs, written
+// and read in one access: a reader waits for the tag it expects, so nothing needs a fence or a separate
+// barrier.  A z is overwritten only after the sum that follows it, to which every reader contributes
+// after its reads.  Sums go over m1 CTAs, then over m2 such groups (a push to each peer's own slots):
+// 2.1 k cycles for up to 16 CTAs and 3.6 k for 144, where an arrival count with release and acquire took
+// 3.8 k and 4.8 k, and polling all partials in one place 9.8 k (every SM then polls the same 37 lines).
 //
 // Co-residency comes from the cooperative launch; every wait has a limit, after which the CTA reports
 // the launch as failed and returns, leaving its system's `done` at 0.  A CTA may have to wait for members
@@ -748,8 +748,8 @@ double iteration_cost(int t, int n, double tile_bytes) {
 }
 
 // The number of CTAs of each system.  A system of up to `alone` tiles is one CTA's work; any other gets
-// all SMs when it is the only one.  In a batch the systems run side by side, each with the CTAs that let all end
-// together (iterations grow like the cells along a side, the cube root of the tiles), as long as
+// all SMs when it is the only one.  In a batch the systems run side by side, each with the CTAs that let
+// all end together (iterations grow like the cells along a side, the cube root of the tiles), as long as
 // their K stays in L2; a larger batch takes several such sets in turn.
 std::vector<int> group_sizes(const std::vector<int>& tiles, int alone, int ncta,
                              double tile_bytes) {

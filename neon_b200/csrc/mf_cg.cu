@@ -372,7 +372,7 @@ constexpr int apply_blocks() {
 // What does not change between iterations is requested before the wait for the kernel ahead.  FP32
 // is held by its 1.7 k instructions per element at 16 to 20 warps per SM, FP64 by the FP64 pipe
 // (1.4 k operations per element, 64 per cycle and SM) at 8 warps.  Per iteration of J2 at 100^3:
-// FP64 450 (assembled K) -> 219 us, FP32 156 -> 141 us.
+// FP64 450 (assembled K) -> 216 us, FP32 156 -> 141 us.
 template <int NPE, int MODEL, typename R>
 __global__ void __launch_bounds__(kThreads<NPE>, apply_blocks<NPE, MODEL, R>())
     k_mf_apply(MfView<R> M, R Kb, const R* z, const R* p, const CgScalars* s) {
@@ -586,10 +586,9 @@ __global__ void __launch_bounds__(kRedThreads) k_mf_p(int N, const float* z, flo
 // q = K p (masked rows 0), p = z + beta p in place (hex8), p.q; the last block forms
 // alpha = (r.z)/(p.q)
 template <int NPE, typename R>
-__global__ void __launch_bounds__(kRedThreads, NPE == 8 && sizeof(R) == 4 ? 8 : 4) k_mf_gather(int N, NodeSums S, const R* ye,
-                                                           const R* z, R* p, R* q,
-                                                           const unsigned char* __restrict__ mask,
-                                                           CgScalars* s, double* partials) {
+__global__ void __launch_bounds__(kRedThreads, NPE == 8 && sizeof(R) == 4 ? 8 : 4)
+    k_mf_gather(int N, NodeSums S, const R* ye, const R* z, R* p, R* q,
+                const unsigned char* __restrict__ mask, CgScalars* s, double* partials) {
     pdl_next();
     pdl_wait();
     if (s->done) return;
@@ -917,7 +916,8 @@ int build_plan(nb2_ctx* c, MfPlan* P) {
     NB2_TRY(allocate(c, &kp, m));
     keys.p = kp;
     auto product_nodes = npe == 8 ? k_product_nodes<8> : k_product_nodes<4>;
-    product_nodes<<<element_grid(c), element_threads(c), 0, c->stream>>>(E, N, c->conn, kp, P->nidx);
+    product_nodes<<<element_grid(c), element_threads(c), 0, c->stream>>>(E, N, c->conn, kp,
+                                                                          P->nidx);
     try {  // its scratch may not fit; no exception may pass the C interface
         thrust::stable_sort_by_key(thrust::cuda::par.on(c->stream), thrust::device_pointer_cast(kp),
                                    thrust::device_pointer_cast(kp + m),
@@ -990,7 +990,8 @@ struct MfRunner {
             }
             if (e == cudaSuccess)
                 e = launch_early(pdl, c->stream, gather_grid(c), (unsigned)kRedThreads, 0,
-                           c->npe == 8 ? k_mf_gather<8, R> : k_mf_gather<4, R>, c->N, sums(c), ye, (const R*)z, p, q, (const unsigned char*)c->mask, c->cgs, c->partials);
+                           c->npe == 8 ? k_mf_gather<8, R> : k_mf_gather<4, R>, c->N, sums(c), ye,
+                           (const R*)z, p, q, (const unsigned char*)c->mask, c->cgs, c->partials);
             if (e == cudaSuccess)
                 e = launch_early(pdl, c->stream, (unsigned)RB, (unsigned)kRedThreads, 0, k_mf_xr<R>,
                            (long long)c->n, x, r, z, (const R*)p, (const R*)q, (const R*)inv,

@@ -257,7 +257,8 @@ int launch_apply(nb2_ctx* c, const double* v, double* y);  // y = K v, FP64 matr
 int launch_element_stiffness(nb2_ctx* c, long long e, double* Ke_dev);  // one dense K_e
 int launch_adjoint_shear(nb2_ctx* c, const double* lam, double* dJdG);
 int launch_force_jvp(nb2_ctx* c, const double* v, double* y);  // exact (d f_int/du) v
-// matrix-free data of the last MODE_STORE pass: FP32 (md, mc) or FP64 (mc), and the element contributions to diag(K)
+// matrix-free data of the last MODE_STORE pass: FP32 (md, mc) or FP64 (mc), and the element contributions
+// to diag(K)
 int launch_mf_setup32(nb2_ctx* c, float* md, float* mc, double* de);
 int launch_mf_setup64(nb2_ctx* c, double* mc, double* de);
 void element_flop_model(const nb2_ctx* c, double* flops_per_element);
